@@ -867,7 +867,8 @@ def test_split_tiles_are_summed_by_their_workers(M, N, K, bn, swiglu):
 
 def test_split_k_on_several_streams_and_under_capture():
     """Launches that overlap on different streams do not share scratch; a stream past the last scratch
-    deals whole tiles; a capture on a stream that has not been used before works and replays."""
+    deals whole tiles; a capture on a stream that has not been used before works (what its replays
+    compute with new inputs: test_captured_split_k_sums_the_partials_of_its_own_replay)."""
     from tridist_b200.ops._gemm_common import gemm_nt
     M, N, K, dt = 128, 4096, 4096, torch.bfloat16
     b = _rand((N, K), 52, dt)
@@ -895,6 +896,90 @@ def test_split_k_on_several_streams_and_under_capture():
     torch.cuda.synchronize()
     for o in outs[:2]:
         assert bool(((o.double() - exact[0]).abs() <= _gemm_bound(a[0], b, exact[0], dt)).all())
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(128, 4096, 4096, 128),      # every tile cut: 32 x 4 slices
+                                      (600, 2304, 4096, 256)])     # CTA pairs
+def test_captured_split_k_sums_the_partials_of_its_own_replay(M, N, K, bn):
+    """A captured GEMM that is cut along K, and two in one graph whose launches share scratch, replayed
+    over other inputs each time, an eager call between two replays, and two graphs of one capture
+    stream replayed at the same time: the bits of the eager call, within the rounding of the 64-bit
+    product."""
+    from tridist_b200.ops._gemm_common import OP_PLAIN, SCHED_NATURAL, gemm_nt
+    dt = torch.bfloat16
+    assert _loaded_native().splitk_dump(dict(op=OP_PLAIN, sched=SCHED_NATURAL, bn=bn, R=1, rank=0, M=M, N=N, K=K,
+                                             by_rounds=1), 148)
+    b = _rand((N, K), 52, dt)
+    a = [torch.zeros((M, K), dtype=dt, device="cuda") for _ in range(3)]
+    outs = [torch.empty((M, N), dtype=dt, device="cuda") for _ in range(3)]
+    gemm_nt(a[0], b, bn=bn)                             # (the first call of a process allocates its status block)
+    torch.cuda.synchronize()
+    capture = torch.cuda.Stream()
+    one, two = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(one, stream=capture):
+        gemm_nt(a[0], b, out=outs[0], bn=bn)
+    with torch.cuda.graph(two, stream=capture):
+        gemm_nt(a[1], b, out=outs[1], bn=bn)
+        gemm_nt(a[2], b, out=outs[2], bn=bn)
+    replay = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for it in range(25):
+        new = [_rand((M, K), 100 + 3 * it + i, dt) for i in range(3)]
+        ref = [gemm_nt(x, b, bn=bn) for x in new]
+        for i in range(3):
+            a[i].copy_(new[i])
+            outs[i].zero_()
+        torch.cuda.synchronize()
+        for graph, s in zip((one, two), replay):
+            with torch.cuda.stream(s):
+                graph.replay()
+        between = gemm_nt(new[0], b, bn=bn)
+        torch.cuda.synchronize()
+        assert torch.equal(between, ref[0])
+        for i in range(3):
+            exact = new[i].double() @ b.double().t()
+            assert torch.equal(outs[i], ref[i]), (it, i)
+            assert bool(((outs[i].double() - exact).abs() <= _gemm_bound(new[i], b, exact, dt)).all()), (it, i)
+    del one, two                                 # their scratch serves the next capture
+    again = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(again, stream=capture):
+        gemm_nt(a[0], b, out=outs[0], bn=bn)
+    outs[0].zero_()
+    again.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], ref[0])
+
+
+def test_split_tiles_meet_again_after_a_launch_that_gave_up(monkeypatch):
+    """Virtual rank 1 does not push, so rank 0's workers leave their cut tiles without having met
+    (20 ms limit); the next launches on the same scratch, over other inputs, sum what they should."""
+    from tridist_b200.ops._gemm_common import gemm_nt
+    from tridist_b200.ops.all_gather_gemm import ag_gemm_emulated, create_ag_gemm_intra_node_context
+    from tridist_b200.parallel.runtime import TriDistError
+    monkeypatch.setenv("TRIDIST_WAIT_TIMEOUT_MS", "20")
+    R, dt = 2, torch.bfloat16
+    w = _emu(R)
+    m_pr, K, N = 256, 4096, 512
+    ctxs = [create_ag_gemm_intra_node_context(m_pr * R, K, dt, dt, r, R, M_PER_CHUNK=128, world=w) for r in range(R)]
+    b = [_rand((N, K), 195 + r, dt) for r in range(R)]
+    c = [torch.empty(m_pr * R, N, dtype=dt, device="cuda") for _ in range(R)]
+    for it in range(3):
+        a = [_rand((m_pr, K), 190 + 2 * it + r, dt) for r in range(R)]
+        if it == 1:
+            ag_gemm_emulated(ctxs, a, b, c, mute_ranks=[1])
+            torch.cuda.synchronize()
+            with pytest.raises(TriDistError, match="all-gather chunk ticket"):
+                w.check()
+            w.clear_status()
+        ag_gemm_emulated(ctxs, a, b, c)
+        plain = gemm_nt(a[0], b[0])
+        torch.cuda.synchronize()
+        w.check()
+        full = torch.cat(a, 0)
+        for r in range(R):
+            exact = full.double() @ b[r].double().t()
+            assert bool(((c[r].double() - exact).abs() <= _gemm_bound(full, b[r], exact, dt)).all()), (it, r)
+        exact = a[0].double() @ b[0].double().t()
+        assert bool(((plain.double() - exact).abs() <= _gemm_bound(a[0], b[0], exact, dt)).all()), it
 
 
 @pytest.mark.parametrize("M,N,K,swiglu", [(128, 512, 1024, False), (384, 2048, 4096, False), (640, 1024, 512, True),

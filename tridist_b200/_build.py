@@ -27,6 +27,7 @@ SOURCES = [
     "bindings.cpp",
     "runtime/symm_heap.cu",
     "runtime/vmm_heap.cu",
+    "runtime/split_scratch.cpp",
     "ops/fused_gemm.cu",
     "ops/elementwise.cu",
     "ops/moe_a2a.cu",

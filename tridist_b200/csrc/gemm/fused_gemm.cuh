@@ -53,6 +53,7 @@
 
 #include "../common/ptx.cuh"
 #include "../common/sync.cuh"
+#include "../runtime/split_scratch.h"
 
 namespace tdb {
 
@@ -65,7 +66,6 @@ constexpr int kEpiWarp0 = 2;
 constexpr int kCommWarp0 = 6;
 constexpr int kCommThreads = 128;
 constexpr int kEpiThreads = 128;
-constexpr int kSkSlots = 160;     // split-K scratch slots (CTAs of a launch)
 constexpr int kMaxSlices = 8;     // K ranges a remainder tile can be cut into
 constexpr int kPushSlots = 12;    // 16 KB pieces in flight per pushing CTA (all-gather)
 
@@ -188,8 +188,8 @@ struct alignas(64) GemmParams {
   int32_t sk_tiles;        // scheduling positions (the last ones) that are cut along K
   int32_t sk_slices;       // K ranges per such position (each on its own worker)
   float* sk_ws;            // [CTA slot][accumulator block][32-column chunk][8][128 threads] x 16 B
-  uint32_t* sk_flags;      // [CTA slot]: epoch of the last partial parked in the slot
-  uint32_t sk_epoch;       // per-launch value, never repeated on a device
+  uint32_t* sk_words;      // [2][kSkSlots], indexed by the CTA slot of a tile's slice 0: slices that have
+                           // parked their partials, slices that wait no more; zero between launches
   int32_t sk_slot_words;   // fp32 words per CTA slot
 
   // ---- OP_AG ----
@@ -565,6 +565,21 @@ __device__ __forceinline__ bool epi_vote(volatile int32_t* flags, bool my_ok, in
 
 __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
+// The slices of a cut tile meet at two words of device memory that a launch finds and leaves at
+// zero: nothing of the meeting comes from the host, so a captured launch can be replayed. A slice
+// arrives when its partials are parked (after the barrier that orders its threads' stores) and
+// leaves when it waits for nobody any more, once each and also when it gave up; the last to leave
+// clears both words, which nobody reads again before the next kernel on this scratch.
+__device__ __forceinline__ void split_arrive(const GemmParams& p, int slot_s0) {
+  atom_add_acq_rel_gpu(p.sk_words + slot_s0, 1u);
+}
+__device__ __forceinline__ void split_leave(const GemmParams& p, int slot_s0, int slices) {
+  if (atom_add_acq_rel_gpu(p.sk_words + kSkSlots + slot_s0, 1u) + 1u == static_cast<uint32_t>(slices)) {
+    st_relaxed_gpu(p.sk_words + slot_s0, 0u);
+    st_relaxed_gpu(p.sk_words + kSkSlots + slot_s0, 0u);
+  }
+}
+
 // Epilogue of a tile that is cut along K and stays on this GPU (all four epilogue warps). Every
 // slice parks the columns that it does not sum itself, waits for the others' and stores the sum
 // of its share: one worker adding all the partials would read slices - 1 whole accumulators
@@ -584,6 +599,7 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
   const int64_t ldc = p.ldc;
   const int slot0 = static_cast<int>(blockIdx.y * gridDim.x);
   const int my_slot = slot0 + static_cast<int>(blockIdx.x);
+  const int slot_s0 = slot0 + (my_worker - slice) * kCtaM + sub;     // slot of slice 0
   bool ok = true;
   if (lane == 0)
     for (int h = 0; ok && h < kMT; ++h)
@@ -591,7 +607,10 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
                      (kMT == 2) ? static_cast<uint32_t>(it & 1) : static_cast<uint32_t>((it >> 1) & 1),
                      env, SITE_TMEM_FULL, h);
   ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
-  if (!epi_vote(s_flags, ok)) return false;
+  if (!epi_vote(s_flags, ok)) {
+    if (etid == 0) split_leave(p, slot_s0, slices);
+    return false;
+  }
   tc_fence_after_sync();
   const bool swiglu = p.epi == EPI_SWIGLU;
   const int n_cols = p.N;
@@ -627,11 +646,10 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
   }
   // the barrier orders all 128 threads' stores before the one release below
   named_bar_sync(2, kEpiThreads);
-  if (etid == 0) st_release_gpu(p.sk_flags + my_slot, p.sk_epoch);
-  const int slot_s0 = slot0 + (my_worker - slice) * kCtaM + sub;     // slot of slice 0
   if (etid == 0) {
-    for (int s = 0; ok && s < slices; ++s)
-      if (s != slice) ok = wait_flag_ge(p.sk_flags + slot_s0 + s * kCtaM, p.sk_epoch, env, SITE_SPLITK, s);
+    split_arrive(p, slot_s0);
+    ok = wait_flag_ge(p.sk_words + slot_s0, static_cast<uint32_t>(slices), env, SITE_SPLITK, slice);
+    split_leave(p, slot_s0, slices);
   }
   if (!epi_vote(s_flags, ok)) return false;
   // The other slices' pieces in the order they are added: block, share unit, (gate, up), slice.
@@ -1149,6 +1167,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
     uint64_t acc_busy = 0, acc_pub = 0, acc_tick = 0, acc_sk = 0, n_tiles_done = 0;
     int it = 0;
     bool alive = true;
+    bool counted_out = false;      // of the cut tile (thread 0)
     WorkIter wit;
     WorkItem wi;
     while (alive && wit.next(wsched, my_worker, p.k_blocks, wi)) {
@@ -1158,6 +1177,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
         alive = split_tile_local<BN, kBf16, kCtaM, kMT>(p, wi.slice, wi.slices, t.m_tile, t.n_tile, tmem_base,
                                                         tmem_full_bar, tmem_empty_bar, s_flags, it, my_worker, sub);
+        counted_out = true;
         if (!alive) break;
         if (prof && etid == 0) {
           acc_sk += globaltimer_ns() - t_sk0;
@@ -1221,7 +1241,12 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
           if (h == kMT - 1) {
             // the barrier orders all 128 threads' stores before the one release below
             named_bar_sync(2, kEpiThreads);
-            if (etid == 0) st_release_gpu(p.sk_flags + my_slot, p.sk_epoch);
+            if (etid == 0) {
+              const int slot_s0 = my_slot - wi.slice * kCtaM;
+              split_arrive(p, slot_s0);
+              split_leave(p, slot_s0, wi.slices);
+            }
+            counted_out = true;
           }
           if (prof && etid == 0) {
             acc_busy += globaltimer_ns() - t_epi0;
@@ -1232,10 +1257,12 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         // slice 0: add the partials of slices 1 .. slices-1 (the next workers) in that order
         const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
         bool ok = true;
-        if (etid == 0) {
-          for (int s = 1; ok && s < wi.slices; ++s)
-            ok = wait_flag_ge(p.sk_flags + slot0 + (my_worker + s) * kCtaM + sub, p.sk_epoch, env,
-                              SITE_SPLITK, s);
+        if (h == 0) {
+          if (etid == 0) {
+            ok = wait_flag_ge(p.sk_words + my_slot, static_cast<uint32_t>(wi.slices - 1), env, SITE_SPLITK, 0);
+            split_leave(p, my_slot, wi.slices);
+          }
+          counted_out = true;
         }
         if (!epi_vote(s_flags, ok)) { alive = false; break; }
         if (prof && etid == 0) acc_sk += globaltimer_ns() - t_sk0;
@@ -1573,6 +1600,13 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
       }
       }   // 128-row blocks of the CTA tile
       ++it;
+    }
+    if (!alive && etid == 0 && !counted_out) {
+      // gave up before the worker's cut tile, if it has one (always its last item): counted out of it here
+      bool cut = wi.slices > 1;
+      while (!cut && wit.next(wsched, my_worker, p.k_blocks, wi)) cut = wi.slices > 1;
+      if (cut && tile_at(p, s_order, wi.pos, sub, bands).valid)
+        split_leave(p, my_slot - wi.slice * kCtaM, wi.slices);
     }
     // staged stores must have read shared memory before the CTA goes away
     if (kStaging && lane == 0) tma_store_wait_all<0>();

@@ -7,7 +7,6 @@
 
 #include <algorithm>
 #include <array>
-#include <atomic>
 #include <mutex>
 #include <stdexcept>
 #include <vector>
@@ -252,67 +251,19 @@ static int grid_for(const GemmPlanDesc& d, GemmParams& p, int max_ctas, int sms)
   return workers * p.cta_m;
 }
 
-// Scratch for the split-K partials: one slot per CTA of a launch (two fp32 accumulators of
-// 128 x 256) and one epoch word per slot, 42 MB in all. Launches on one stream follow one another, launches on
-// two streams may overlap: each stream has a scratch of its own, allocated on its first use and
-// never freed (a captured graph keeps the address). Past kSkStreams streams of a device there is
-// none, and the launch deals whole tiles.
-constexpr int64_t kSkSlotWords = 2ll * BM * 256;
-constexpr int kSkStreams = 8;
-struct SkScratch {
-  cudaStream_t stream = nullptr;
-  float* ws = nullptr;
-  uint32_t* flags = nullptr;
-};
-static std::mutex g_sk_mu;
-static bool sk_scratch(cudaStream_t stream, SkScratch* out) {
-  static SkScratch per_dev[64][kSkStreams];
-  int dev = 0;
-  check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lk(g_sk_mu);
-  SkScratch* s = per_dev[dev & 63];
-  for (int i = 0; i < kSkStreams; ++i, ++s) {
-    if (s->ws != nullptr && s->stream != stream) continue;
-    if (s->ws == nullptr) {
-      // the stream may be capturing: allocate and clear outside of it
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-      check(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-      SkScratch fresh;
-      fresh.stream = stream;
-      cudaStream_t side = nullptr;
-      cudaError_t e = cudaMalloc(&fresh.ws, kSkSlots * kSkSlotWords * sizeof(float));
-      if (e == cudaSuccess) e = cudaMalloc(&fresh.flags, kSkSlots * sizeof(uint32_t));
-      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaMemsetAsync(fresh.flags, 0, kSkSlots * sizeof(uint32_t), side);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(side);
-      if (side) cudaStreamDestroy(side);
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      if (e != cudaSuccess) {
-        cudaFree(fresh.ws);
-        cudaFree(fresh.flags);
-        check(e, "split-K scratch");
-      }
-      *s = fresh;
-    }
-    *out = *s;
-    return true;
-  }
-  return false;
-}
-static std::atomic<uint32_t> g_sk_epoch{0};
-
-// The scratch of `stream` into a launch's parameters; whole tiles where there is none.
-static void bind_sk_scratch(GemmParams& p, cudaStream_t stream, uint32_t epoch) {
-  if (p.sk_tiles == 0) return;
-  SkScratch sc;
-  if (!sk_scratch(stream, &sc)) {
+// Scratch of the stream (or of the graph it is being captured into) into a launch's parameters;
+// whole tiles where there is none. What comes back is held until the launch is in the stream.
+static SplitScratch bind_sk_scratch(GemmParams& p, int slots, cudaStream_t stream) {
+  if (p.sk_tiles == 0) return {};
+  SplitScratch sc = split_scratch(stream, slots * static_cast<int64_t>(p.sk_slot_words));
+  if (sc.partials == nullptr) {
     p.sk_tiles = 0;
     p.sk_slices = 1;
-    return;
+    return sc;
   }
-  p.sk_ws = sc.ws;
-  p.sk_flags = sc.flags;
-  p.sk_epoch = epoch;
+  p.sk_ws = sc.partials;
+  p.sk_words = sc.words;
+  return sc;
 }
 
 std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& d, int sms) {
@@ -671,7 +622,7 @@ void gemm_plan_launch(int64_t id, uint32_t round, int parity, int64_t order_tabl
   p.skip_comm = flags & 1;
   p.comm_only = (flags >> 1) & 1;
   p.publish_only = (flags >> 2) & 1;
-  bind_sk_scratch(p, stream, ++g_sk_epoch);
+  const SplitScratch scratch = bind_sk_scratch(p, p.sk_tiles * p.sk_slices * p.cta_m, stream);
   const bool staging = plan_uses_staging(p);
 #define TDB_LAUNCH(BN_, PAIR_)                                                              \
   do {                                                                                      \
@@ -735,7 +686,6 @@ void gemm_plans_launch_emulated(const std::vector<int64_t>& ids, uint32_t round,
   if (vr < 1 || vr > kMaxRanks) throw std::runtime_error("tridist_b200: bad emulated rank count");
   GemmPlan* first = find_plan(ids[0]);
   std::vector<GemmParams> host(vr);
-  const uint32_t epoch = ++g_sk_epoch;
   int grid_x = (num_sms() / vr) / first->cta_m * first->cta_m;
   for (int i = 0; i < vr; ++i) {
     GemmPlan* pl = find_plan(ids[i]);
@@ -753,7 +703,8 @@ void gemm_plans_launch_emulated(const std::vector<int64_t>& ids, uint32_t round,
       host[i].sk_slices = 1;
     }
   }
-  for (int i = 0; i < vr; ++i) bind_sk_scratch(host[i], stream, epoch);
+  std::vector<SplitScratch> scratch;      // (one scratch: the ranks have slots of their own in it)
+  for (int i = 0; i < vr; ++i) scratch.push_back(bind_sk_scratch(host[i], grid_x * vr, stream));
   if (!first->dev_params)
     check(cudaMalloc(&first->dev_params, sizeof(GemmParams) * kMaxRanks), "cudaMalloc(params)");
   check(cudaMemcpyAsync(first->dev_params, host.data(), sizeof(GemmParams) * vr,
