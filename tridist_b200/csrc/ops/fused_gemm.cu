@@ -251,16 +251,11 @@ static int grid_for(const GemmPlanDesc& d, GemmParams& p, int max_ctas, int sms)
   return workers * p.cta_m;
 }
 
-// Scratch of the stream (or of the graph it is being captured into) into a launch's parameters;
-// whole tiles where there is none. What comes back is held until the launch is in the stream.
+// Scratch of the stream (or of the graph it is being captured into) into a launch's parameters. What
+// comes back is held until the launch is in the stream.
 static SplitScratch bind_sk_scratch(GemmParams& p, int slots, cudaStream_t stream) {
   if (p.sk_tiles == 0) return {};
   SplitScratch sc = split_scratch(stream, slots * static_cast<int64_t>(p.sk_slot_words));
-  if (sc.partials == nullptr) {
-    p.sk_tiles = 0;
-    p.sk_slices = 1;
-    return sc;
-  }
   p.sk_ws = sc.partials;
   p.sk_words = sc.words;
   return sc;

@@ -6,6 +6,7 @@
 // their last replay are done. The block then serves the next capture, or is freed.
 #include "split_scratch.h"
 
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <cuda_runtime.h>
 
 #include <map>
@@ -157,29 +158,59 @@ SplitScratch of_capture(int dev, cudaStream_t stream, unsigned long long id, cud
 }
 
 // ---- eager launches ------------------------------------------------------------------------------
-// One block per stream, allocated on its first use and never freed. Past kSkStreams streams of a
-// device there is none, and the launch deals whole tiles.
-constexpr int kSkStreams = 8;
-constexpr int64_t kEagerBytes = kWordBytes + kSkSlots * 2ll * 128 * 256 * 4;
+// A block per stream, kept from call to call, from torch's allocator: memory allocated on a stream goes
+// back to that stream's work only, so a block can be dropped while launches that use it are pending.
+// The streams used last keep theirs (38 MB at most); a program that goes round more of them pays for
+// an allocation from the cache and a clear of the words (a 2 KB memset) on its calls.
+constexpr size_t kStreamBlocks = 16;
 
-SplitScratch of_stream(int dev, cudaStream_t stream) {
-  struct Slot {
-    cudaStream_t stream = nullptr;
-    Block block;
-  };
-  static std::mutex mu;
-  static Slot per_dev[64][kSkStreams];
-  std::lock_guard<std::mutex> lk(mu);
-  for (Slot& s : per_dev[dev & 63]) {
-    if (s.block.base != nullptr && s.stream != stream) continue;
-    if (s.block.base == nullptr) {
-      OutsideCapture guard;               // (another stream may be capturing)
-      s.block = new_block(kEagerBytes);
-      s.stream = stream;
+struct StreamBlock {
+  int dev = -1;
+  unsigned long long stream = 0;          // id: a handle can be given out again while old work is pending
+  uint64_t used = 0;
+  int64_t bytes = 0;
+  std::shared_ptr<void> mem;
+};
+struct StreamBlocks {
+  std::mutex mu;
+  uint64_t clock = 0;
+  std::vector<StreamBlock> blocks;
+};
+
+SplitScratch of_stream(int dev, cudaStream_t stream, int64_t bytes) {
+  static StreamBlocks& sb = *new StreamBlocks;            // not destroyed under a driver that is gone
+  unsigned long long id = 0;
+  check(cudaStreamGetId(stream, &id), "cudaStreamGetId");
+  std::lock_guard<std::mutex> lk(sb.mu);
+  StreamBlock* b = nullptr;
+  for (StreamBlock& x : sb.blocks)
+    if (x.stream == id && x.dev == dev) b = &x;
+  if (b == nullptr) {
+    if (sb.blocks.size() < kStreamBlocks) {
+      sb.blocks.emplace_back();
+      b = &sb.blocks.back();
+    } else {
+      b = &sb.blocks[0];
+      for (StreamBlock& x : sb.blocks)
+        if (x.used < b->used) b = &x;
+      *b = StreamBlock{};
     }
-    return view(s.block);
+    b->dev = dev;
+    b->stream = id;
   }
-  return {};
+  b->used = ++sb.clock;
+  if (b->bytes < bytes) {
+    b->bytes = 0;
+    b->mem.reset();
+    std::shared_ptr<void> mem(c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(static_cast<size_t>(bytes), stream),
+                              c10::cuda::CUDACachingAllocator::raw_delete);
+    check(cudaMemsetAsync(mem.get(), 0, kWordBytes, stream), "split-K scratch");
+    b->mem = std::move(mem);
+    b->bytes = bytes;
+  }
+  SplitScratch s = view({static_cast<uint8_t*>(b->mem.get()), b->bytes});
+  s.hold = b->mem;
+  return s;
 }
 
 }  // namespace
@@ -187,6 +218,7 @@ SplitScratch of_stream(int dev, cudaStream_t stream) {
 SplitScratch split_scratch(cudaStream_t stream, int64_t words) {
   int dev = 0;
   check(cudaGetDevice(&dev), "cudaGetDevice");
+  const int64_t bytes = kWordBytes + words * static_cast<int64_t>(sizeof(float));
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
   cudaGraph_t graph = nullptr;
@@ -195,8 +227,8 @@ SplitScratch split_scratch(cudaStream_t stream, int64_t words) {
   if (status == cudaStreamCaptureStatusInvalidated)
     throw std::runtime_error("tridist_b200: the capture of this stream has failed");
   if (status == cudaStreamCaptureStatusActive)
-    return of_capture(dev, stream, id, graph, kWordBytes + words * static_cast<int64_t>(sizeof(float)));
-  return of_stream(dev, stream);
+    return of_capture(dev, stream, id, graph, bytes);
+  return of_stream(dev, stream, bytes);
 }
 
 }  // namespace tdb

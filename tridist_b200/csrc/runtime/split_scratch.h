@@ -10,7 +10,7 @@ namespace tdb {
 constexpr int kSkSlots = 160;     // CTAs of a launch that can take part in a cut tile
 
 struct SplitScratch {
-  float* partials = nullptr;      // nullptr = none to be had: deal whole tiles
+  float* partials = nullptr;
   uint32_t* words = nullptr;      // [2][kSkSlots], zero between launches
   std::shared_ptr<void> hold;     // keeps the memory until the launch is in the stream
 };
