@@ -464,6 +464,15 @@ def test_split_k_slices_are_used(monkeypatch):
         assert cuts and all(2 <= c[3] <= 8 for c in cuts)
 
 
+def test_gemm_variants_keep_their_tile_loop_in_registers():
+    """Local memory per thread (stack and spills) of every variant: 32 bytes are the producer's table of
+    observed shards, the rest are spills, at most what they were before tiles cut along K were summed
+    by all their workers (80, 112 and 176 bytes)."""
+    for bn, bf16, pair, staging, mt, regs, local in _loaded_native().gemm_variants():
+        limit = 32 if not staging else 208 if mt == 2 else 144 if bn == 256 else 112
+        assert regs <= 168 and local <= limit, (bn, bf16, pair, staging, mt, local)
+
+
 @pytest.mark.parametrize("tiles", ["single", "pair", "wide"])
 def test_fused_ops_emulated_many_tiles_per_cta(tiles, monkeypatch):
     """Two virtual ranks, 8 CTAs each, 2048-row problems: AG (pushing CTAs join late), RS and both

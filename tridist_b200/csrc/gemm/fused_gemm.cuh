@@ -408,6 +408,17 @@ __host__ __device__ __forceinline__ int remainder_positions(int positions, int w
 struct WorkItem {
   int pos, kb0, kb1, slice, slices;
 };
+// The worker's K range of a cut tile, if it has one. It comes after all of the worker's whole tiles.
+__host__ __device__ __forceinline__ bool cut_item(const WorkerSchedule& w, int my_worker, int k_blocks, WorkItem& wi) {
+  if (my_worker >= w.sk_tiles * w.sk_slices) return false;
+  const int t = my_worker / w.sk_slices, s = my_worker - t * w.sk_slices;
+  wi.pos = w.dp_positions + t;
+  wi.kb0 = static_cast<int>(static_cast<long long>(s) * k_blocks / w.sk_slices);
+  wi.kb1 = static_cast<int>(static_cast<long long>(s + 1) * k_blocks / w.sk_slices);
+  wi.slice = s;
+  wi.slices = w.sk_slices;
+  return true;
+}
 struct WorkIter {
   int i = 0;
   bool sk_seen = false;
@@ -420,14 +431,7 @@ struct WorkIter {
       return true;
     }
     sk_seen = true;
-    if (my_worker >= w.sk_tiles * w.sk_slices) return false;
-    const int t = my_worker / w.sk_slices, s = my_worker - t * w.sk_slices;
-    wi.pos = w.dp_positions + t;
-    wi.kb0 = static_cast<int>(static_cast<long long>(s) * k_blocks / w.sk_slices);
-    wi.kb1 = static_cast<int>(static_cast<long long>(s + 1) * k_blocks / w.sk_slices);
-    wi.slice = s;
-    wi.slices = w.sk_slices;
-    return true;
+    return cut_item(w, my_worker, k_blocks, wi);
   }
 };
 
@@ -580,15 +584,16 @@ __device__ __forceinline__ void split_leave(const GemmParams& p, int slot_s0, in
   }
 }
 
-// Epilogue of a tile that is cut along K and stays on this GPU (all four epilogue warps). Every
-// slice parks the columns that it does not sum itself, waits for the others' and stores the sum
-// of its share: one worker adding all the partials would read slices - 1 whole accumulators
-// through one SM (128 tokens against 7168 x 8192 and 8192 x 3584 weights, five and two slices:
-// 80 us that way, 63 us shared). Scratch layout of a slot: [accumulator block][32-column chunk]
-// [16-byte piece][thread]. Not inlined: its registers would be taken from the other epilogues'
-// column loops.
+// Epilogue of a worker's K range of a cut tile (all four epilogue warps). Where the tile goes to other
+// ranks (`local` false) slices 1 .. slices-1 park their accumulator here, for slice 0 to add. Where it
+// stays on this GPU every slice parks the columns that it does not sum itself, waits for the others'
+// and stores the sum of its share: one worker adding all the partials would read slices - 1 whole
+// accumulators through one SM (128 tokens against 7168 x 8192 and 8192 x 3584 weights, five and two
+// slices: 80 us that way, 68 us shared). Scratch layout of a slot: [accumulator block][32-column chunk]
+// [16-byte piece][thread]. Called behind the tile loop: a call inside it kept the loop's state live
+// across this and made every variant of the kernel spill (400 to 1300 bytes of loads).
 template <int BN, bool kBf16, int kCtaM, int kMT>
-__device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, int slices, int m_tile, int n_tile,
+__device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int slice, int slices, int m_tile, int n_tile,
                                               uint32_t tmem_base, uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar,
                                               volatile int32_t* s_flags, int it, int my_worker, int sub) {
   const WaitEnv& env = p.env;
@@ -607,10 +612,7 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
                      (kMT == 2) ? static_cast<uint32_t>(it & 1) : static_cast<uint32_t>((it >> 1) & 1),
                      env, SITE_TMEM_FULL, h);
   ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
-  if (!epi_vote(s_flags, ok)) {
-    if (etid == 0) split_leave(p, slot_s0, slices);
-    return false;
-  }
+  if (!epi_vote(s_flags, ok)) return false;
   tc_fence_after_sync();
   const bool swiglu = p.epi == EPI_SWIGLU;
   const int n_cols = p.N;
@@ -635,7 +637,7 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
 #pragma unroll 1
   for (int hc = 0; hc < kMT * (BN / 32); ++hc) {
     const int u = swiglu ? hc % (BN / 64) : hc % (BN / 32);
-    if (u >= u_lo && u < u_hi) continue;
+    if (local && u >= u_lo && u < u_hi) continue;
     uint32_t r[32];
     tmem_ld_32x32b_x32(tq + hc * 32, r);      // (accumulator block 1 follows block 0)
     tmem_ld_wait();
@@ -646,10 +648,13 @@ __device__ __noinline__ bool split_tile_local(const GemmParams& p, int slice, in
   }
   // the barrier orders all 128 threads' stores before the one release below
   named_bar_sync(2, kEpiThreads);
+  if (etid == 0) split_arrive(p, slot_s0);
+  if (!local) {
+    release();
+    return true;
+  }
   if (etid == 0) {
-    split_arrive(p, slot_s0);
     ok = wait_flag_ge(p.sk_words + slot_s0, static_cast<uint32_t>(slices), env, SITE_SPLITK, slice);
-    split_leave(p, slot_s0, slices);
   }
   if (!epi_vote(s_flags, ok)) return false;
   // The other slices' pieces in the order they are added: block, share unit, (gate, up), slice.
@@ -1164,27 +1169,57 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
     // scratch slots of the split-K partials are indexed by the CTA's place in the launch
     const int slot0 = static_cast<int>(blockIdx.y * gridDim.x);
     const int my_slot = slot0 + static_cast<int>(blockIdx.x);
-    uint64_t acc_busy = 0, acc_pub = 0, acc_tick = 0, acc_sk = 0, n_tiles_done = 0;
+    // (the sums of the accounting stand in its buffer: registers of theirs would be spilled with it off)
+    if (prof && etid == 0) {
+      prof[PROF_EPI_BUSY] = prof[PROF_EPI_PUBLISH] = prof[PROF_EPI_TICKET_WAIT] = 0;
+      prof[PROF_EPI_TILES] = prof[PROF_SK_WAIT] = 0;
+    }
+    const bool split_local = !multi || p.op == OP_PLAIN || p.op == OP_AG;   // a cut tile stays on this GPU
     int it = 0;
     bool alive = true;
-    bool counted_out = false;      // of the cut tile (thread 0)
     WorkIter wit;
     WorkItem wi;
     while (alive && wit.next(wsched, my_worker, p.k_blocks, wi)) {
       const TileCoord t = tile_at(p, s_order, wi.pos, sub, bands);
       if (!t.valid) continue;
-      if (wi.slices > 1 && (!multi || p.op == OP_PLAIN || p.op == OP_AG)) {
+      if (wi.slices > 1 && (split_local || wi.slice > 0)) break;      // done behind the loop
+      if (wi.slices > 1) {
+        // slice 0 of a tile for other ranks adds the partials of slices 1 .. slices-1 (the next
+        // workers) in that order and goes on as with a whole tile
         const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
-        alive = split_tile_local<BN, kBf16, kCtaM, kMT>(p, wi.slice, wi.slices, t.m_tile, t.n_tile, tmem_base,
-                                                        tmem_full_bar, tmem_empty_bar, s_flags, it, my_worker, sub);
-        counted_out = true;
-        if (!alive) break;
-        if (prof && etid == 0) {
-          acc_sk += globaltimer_ns() - t_sk0;
-          n_tiles_done += kMT;
+        bool ok = true;
+        if (lane == 0)
+          for (int h = 0; ok && h < kMT; ++h)
+            ok = wait_mbar(&tmem_full_bar[(kMT == 2) ? h : (it & 1)],
+                           (kMT == 2) ? static_cast<uint32_t>(it & 1) : static_cast<uint32_t>((it >> 1) & 1),
+                           env, SITE_TMEM_FULL, h);
+        if (ok && etid == 0)
+          ok = wait_flag_ge(p.sk_words + my_slot, static_cast<uint32_t>(wi.slices - 1), env, SITE_SPLITK, 0);
+        if (!epi_vote(s_flags, ok)) { alive = false; break; }
+        if (prof && etid == 0) prof[PROF_SK_WAIT] += globaltimer_ns() - t_sk0;
+        tc_fence_after_sync();
+        const uint32_t tq = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                            static_cast<uint32_t>((kMT == 2) ? 0 : (it & 1) * BN);
+#pragma unroll 1
+        for (int c = 0; c < kMT * (BN / 32); ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(tq + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll 1
+          for (int s = 1; s < wi.slices; ++s) {
+            const float* src = p.sk_ws + (my_slot + s * kCtaM) * static_cast<int64_t>(p.sk_slot_words) + etid * 4;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+              const uint4 x = ld_global_cg_v4(src + (c * 8 + v) * (kEpiThreads * 4));
+              r[v * 4 + 0] = __float_as_uint(__uint_as_float(r[v * 4 + 0]) + __uint_as_float(x.x));
+              r[v * 4 + 1] = __float_as_uint(__uint_as_float(r[v * 4 + 1]) + __uint_as_float(x.y));
+              r[v * 4 + 2] = __float_as_uint(__uint_as_float(r[v * 4 + 2]) + __uint_as_float(x.z));
+              r[v * 4 + 3] = __float_as_uint(__uint_as_float(r[v * 4 + 3]) + __uint_as_float(x.w));
+            }
+          }
+          tmem_st_32x32b_x32(tq + c * 32, r);
         }
-        ++it;
-        continue;
+        tmem_st_wait();
       }
       for (int h = 0; alive && h < kMT; ++h) {
       const int buf = (kMT == 2) ? h : (it & 1);
@@ -1221,72 +1256,6 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         }
         released = true;
       };
-
-      // ---- split-K: slices other than 0 park their fp32 accumulator and are done ----------
-      if (wi.slices > 1) {
-        // layout of a slot: [accumulator block][32-column chunk][16-byte piece][thread]
-        if (wi.slice > 0) {
-          float* dst = p.sk_ws + static_cast<int64_t>(my_slot) * p.sk_slot_words + h * (BM * BN);
-#pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x32(taddr + c * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              st_global_v4(dst + ((c * 8 + v) * kEpiThreads + etid) * 4,
-                           make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]));
-          }
-          release_acc();
-          if (h == kMT - 1) {
-            // the barrier orders all 128 threads' stores before the one release below
-            named_bar_sync(2, kEpiThreads);
-            if (etid == 0) {
-              const int slot_s0 = my_slot - wi.slice * kCtaM;
-              split_arrive(p, slot_s0);
-              split_leave(p, slot_s0, wi.slices);
-            }
-            counted_out = true;
-          }
-          if (prof && etid == 0) {
-            acc_busy += globaltimer_ns() - t_epi0;
-            ++n_tiles_done;
-          }
-          continue;
-        }
-        // slice 0: add the partials of slices 1 .. slices-1 (the next workers) in that order
-        const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
-        bool ok = true;
-        if (h == 0) {
-          if (etid == 0) {
-            ok = wait_flag_ge(p.sk_words + my_slot, static_cast<uint32_t>(wi.slices - 1), env, SITE_SPLITK, 0);
-            split_leave(p, my_slot, wi.slices);
-          }
-          counted_out = true;
-        }
-        if (!epi_vote(s_flags, ok)) { alive = false; break; }
-        if (prof && etid == 0) acc_sk += globaltimer_ns() - t_sk0;
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + c * 32, r);
-          tmem_ld_wait();
-          for (int s = 1; s < wi.slices; ++s) {
-            const float* src = p.sk_ws +
-                static_cast<int64_t>(slot0 + (my_worker + s) * kCtaM + sub) * p.sk_slot_words + h * (BM * BN);
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              const uint4 x = ld_global_cg_v4(src + ((c * 8 + v) * kEpiThreads + etid) * 4);
-              r[v * 4 + 0] = __float_as_uint(__uint_as_float(r[v * 4 + 0]) + __uint_as_float(x.x));
-              r[v * 4 + 1] = __float_as_uint(__uint_as_float(r[v * 4 + 1]) + __uint_as_float(x.y));
-              r[v * 4 + 2] = __float_as_uint(__uint_as_float(r[v * 4 + 2]) + __uint_as_float(x.z));
-              r[v * 4 + 3] = __float_as_uint(__uint_as_float(r[v * 4 + 3]) + __uint_as_float(x.w));
-            }
-          }
-          tmem_st_32x32b_x32(taddr + c * 32, r);
-        }
-        tmem_st_wait();
-      }
 
       // ---- routing: which rank keeps this lane's row / this tile --------------
       int owner = p.rank;
@@ -1463,8 +1432,8 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
       }
 
       if (prof && etid == 0) {
-        acc_pub += t_pub1 - t_pub0;
-        acc_tick += globaltimer_ns() - t_pub1;
+        prof[PROF_EPI_PUBLISH] += t_pub1 - t_pub0;
+        prof[PROF_EPI_TICKET_WAIT] += globaltimer_ns() - t_pub1;
       }
       // ---- phase 3: final values of the rows / tile this rank keeps ---------------
       const bool finalizes =
@@ -1595,27 +1564,30 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
 
       if (!released) release_acc();
       if (prof && etid == 0) {
-        acc_busy += globaltimer_ns() - t_epi0;
-        ++n_tiles_done;
+        prof[PROF_EPI_BUSY] += globaltimer_ns() - t_epi0;
+        ++prof[PROF_EPI_TILES];
       }
       }   // 128-row blocks of the CTA tile
       ++it;
     }
-    if (!alive && etid == 0 && !counted_out) {
-      // gave up before the worker's cut tile, if it has one (always its last item): counted out of it here
-      bool cut = wi.slices > 1;
-      while (!cut && wit.next(wsched, my_worker, p.k_blocks, wi)) cut = wi.slices > 1;
-      if (cut && tile_at(p, s_order, wi.pos, sub, bands).valid)
-        split_leave(p, my_slot - wi.slice * kCtaM, wi.slices);
+    // The cut tile is a worker's last item. Behind the loop nothing else is live, so that its registers
+    // are not taken from the whole tiles' epilogue.
+    if (cut_item(wsched, my_worker, p.k_blocks, wi)) {
+      const TileCoord t = tile_at(p, s_order, wi.pos, sub, bands);
+      if (alive && t.valid && (split_local || wi.slice > 0)) {
+        const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
+        if (split_tile<BN, kBf16, kCtaM, kMT>(p, split_local, wi.slice, wi.slices, t.m_tile, t.n_tile, tmem_base,
+                                              tmem_full_bar, tmem_empty_bar, s_flags, it, my_worker, sub) &&
+            prof && etid == 0) {
+          prof[PROF_SK_WAIT] += globaltimer_ns() - t_sk0;
+          prof[PROF_EPI_TILES] += kMT;
+        }
+      }
+      if (t.valid && etid == 0) split_leave(p, my_slot - wi.slice * kCtaM, wi.slices);
     }
     // staged stores must have read shared memory before the CTA goes away
     if (kStaging && lane == 0) tma_store_wait_all<0>();
     if (prof && etid == 0) {
-      prof[PROF_EPI_BUSY] = acc_busy;
-      prof[PROF_EPI_PUBLISH] = acc_pub;
-      prof[PROF_EPI_TICKET_WAIT] = acc_tick;
-      prof[PROF_EPI_TILES] = n_tiles_done;
-      prof[PROF_SK_WAIT] = acc_sk;
       prof[PROF_EPI_DONE_AT] = globaltimer_ns() - t_kernel0;
     }
   }

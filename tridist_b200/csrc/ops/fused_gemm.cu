@@ -579,6 +579,29 @@ static int resident_ctas_of(const GemmPlan& plan) {
 }
 
 template <int BN, bool kBf16, int kCtaM, bool kStaging, int kMT>
+static std::array<int, 7> variant_info() {
+  cudaFuncAttributes at;
+  check(cudaFuncGetAttributes(&at, fused_gemm_kernel<BN, kBf16, kCtaM, kStaging, kMT>), "cudaFuncGetAttributes");
+  return {BN, kBf16, kCtaM, kStaging, kMT, at.numRegs, static_cast<int>(at.localSizeBytes)};
+}
+
+std::vector<std::array<int, 7>> gemm_variants() {
+  std::vector<std::array<int, 7>> v;
+#define TDB_INFO(BN_, PAIR_, STAGING_, MT_)                        \
+  v.push_back(variant_info<BN_, false, PAIR_, STAGING_, MT_>());   \
+  v.push_back(variant_info<BN_, true, PAIR_, STAGING_, MT_>())
+  TDB_INFO(128, 1, false, 1);
+  TDB_INFO(128, 1, true, 1);
+  TDB_INFO(256, 1, false, 1);
+  TDB_INFO(256, 1, true, 1);
+  TDB_INFO(256, 2, false, 1);
+  TDB_INFO(256, 2, true, 1);
+  TDB_INFO(256, 2, true, 2);
+#undef TDB_INFO
+  return v;
+}
+
+template <int BN, bool kBf16, int kCtaM, bool kStaging, int kMT>
 static void launch_one(const GemmParams& p, int grid_x, cudaStream_t stream) {
   set_attr_once<BN, kBf16, kCtaM, kStaging, kMT>();
   cudaLaunchConfig_t cfg = {};

@@ -119,6 +119,9 @@ struct PlanExtents {
 // compute against the given extents. Returns one sentence per violation (empty = consistent).
 std::vector<std::string> plan_check(const GemmPlanDesc& d, const PlanExtents& e, int sms);
 
+// Every variant of the kernel: {BN, bf16, CTAs per pair, staging, 128-row blocks per CTA, registers per
+// thread, bytes of local memory per thread (stack and spills)}.
+std::vector<std::array<int, 7>> gemm_variants();
 int64_t launch_count();
 void launch_count_add(int64_t n);
 
