@@ -71,6 +71,27 @@ def test_gemm_swiglu_epilogue_and_kernel():
     assert (got.float() - exp).abs().max().item() < 1e-2
 
 
+@pytest.mark.parametrize("M,I", [(64, 264), (2112, 1408)])
+def test_swiglu_reads_what_the_gemm_in_front_of_it_wrote(M, I):
+    """The activation starts under the tail of the GEMM that writes its input, over the same buffer with other
+    contents each time and without a synchronisation: the bits of a call on the finished buffer."""
+    from tridist_b200.ops import swiglu
+    from tridist_b200.ops._gemm_common import gemm_nt
+    K, dt = 512, torch.bfloat16
+    w = _rand((2 * I, K), 4, dt)
+    h = torch.empty((M, 2 * I), dtype=dt, device="cuda")
+    xs = [_rand((M, K), 5 + i, dt) for i in range(8)]
+    got = []
+    for x in xs:
+        gemm_nt(x, w, out=h)
+        got.append(swiglu(h))
+    torch.cuda.synchronize()
+    for x, g in zip(xs, got):
+        ref = gemm_nt(x, w)
+        torch.cuda.synchronize()
+        assert torch.equal(g, swiglu(ref))
+
+
 def test_public_api_single_rank():
     """R = 1 degenerates: every op collapses to the local GEMM / permutation."""
     from tridist_b200.ops import (ag_gemm_intra_node, create_ag_gemm_intra_node_context,

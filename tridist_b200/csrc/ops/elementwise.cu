@@ -49,7 +49,9 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   griddep_wait();
   griddep_launch();
-  // two independent 16-byte gate/up pairs per iteration keep four loads in flight per thread
+  // two independent 16-byte gate/up pairs per iteration keep four loads in flight per thread; not through
+  // the read-only path, which wants data that nobody writes while this kernel lives, and it is launched
+  // while the GEMM in front of it still writes h
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += 2 * stride) {
     const int64_t i2 = i + stride;
     const bool two = i2 < total;
@@ -57,10 +59,10 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__
     const int64_t r1 = two ? i2 / vec_per_row : r0, v1 = two ? i2 - r1 * vec_per_row : v0;
     const uint8_t* row0 = h + r0 * ldh * 2;
     const uint8_t* row1 = h + r1 * ldh * 2;
-    const uint4 g0 = ld_global_nc_v4(row0 + v0 * 16);
-    const uint4 u0 = ld_global_nc_v4(row0 + inter * 2 + v0 * 16);
-    const uint4 g1 = ld_global_nc_v4(row1 + v1 * 16);
-    const uint4 u1 = ld_global_nc_v4(row1 + inter * 2 + v1 * 16);
+    const uint4 g0 = ld_global_cg_v4(row0 + v0 * 16);
+    const uint4 u0 = ld_global_cg_v4(row0 + inter * 2 + v0 * 16);
+    const uint4 g1 = ld_global_cg_v4(row1 + v1 * 16);
+    const uint4 u1 = ld_global_cg_v4(row1 + inter * 2 + v1 * 16);
     uint4 o;
     o.x = swiglu2<kBf16>(g0.x, u0.x);
     o.y = swiglu2<kBf16>(g0.y, u0.y);
