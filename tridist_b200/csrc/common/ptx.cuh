@@ -107,7 +107,9 @@ __device__ __forceinline__ void fence_acq_rel_gpu() {
 // predecessor in the stream drains; it must not touch global memory (L2 requests apart) before
 // griddep_wait, which returns when the predecessor has completed and its writes are visible.
 // griddep_launch comes after it, so that "my predecessor started its successor" implies that all
-// earlier kernels of the stream are complete. Without the attribute neither does anything.
+// earlier kernels of the stream are complete. griddep_wait does nothing in a kernel launched without the
+// attribute; griddep_launch does: it releases a successor that has it. So kernels that wait for peers
+// call neither, or a local successor would hold SMs for as long as they wait.
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() {

@@ -822,7 +822,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
   else __syncthreads();
   tc_fence_after_sync();
   griddep_wait();      // (local launches only: the prologue above ran under the previous kernel's tail)
-  griddep_launch();
+  if (p.R == 1) griddep_launch();      // (a kernel that waits for peers keeps its successor off the SMs)
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
   const int bands = *reinterpret_cast<volatile int32_t*>(s_tab);
 

@@ -91,7 +91,7 @@ moe_meta_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict__ 
   if (tid == 0) s_ok = 1;
   __syncthreads();
   griddep_wait();
-  griddep_launch();
+  if (d.R == 1) griddep_launch();
   const int pairs = d.T * d.topk;
   const int lo = cta * d.meta_chunk, hi = min(pairs, lo + d.meta_chunk);
   for (int i = lo + tid; i < hi; i += 2 * kMetaThreads) {
@@ -199,7 +199,7 @@ moe_dispatch_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restric
   const int64_t units = static_cast<int64_t>(d.T) * runs;
   const int topk = d.topk;
   griddep_wait();
-  griddep_launch();
+  if (d.R == 1) griddep_launch();
   for (int64_t unit = static_cast<int64_t>(cta) * (kRowThreads / 32) + warp; unit < units;
        unit += static_cast<int64_t>(ncta) * (kRowThreads / 32)) {
     const int t = static_cast<int>(unit / runs);
@@ -332,7 +332,7 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
   mbar_fence_init();
   __syncthreads();
   griddep_wait();
-  griddep_launch();
+  if (d.R == 1) griddep_launch();
   if (d.R > 1) {
     if (cta == 0 && tid < d.R) {
       __threadfence_system();
