@@ -751,6 +751,27 @@ def test_gemm_ar_rd_emulated(R):
             assert torch.equal(c_list[r], c_list[0]), "all ranks must hold bit-identical results"
 
 
+def test_gemm_ar_rd_keeps_its_tiles(monkeypatch):
+    """The panel GEMMs of several ranks take neither the tile rules of one rank nor its overlapped start."""
+    from tridist_b200.ops.gemm_ar_rd import create_gemm_ar_rd_context, gemm_ar_rd_emulated
+    C = _loaded_native()
+    made = []
+    create = C.gemm_plan_create
+    monkeypatch.setattr(C, "gemm_plan_create", lambda d: (made.append(dict(d)), create(d))[1])
+    R, M, N, K, dt = 2, 512, 8192, 8192, torch.bfloat16
+    w = _emu(R)
+    ctxs = [create_gemm_ar_rd_context(M, N, dt, dt, r, R, chunk_rows=256, stage_slots=2, world=w) for r in range(R)]
+    a, b = [_rand((M, K), 31 + r, dt) for r in range(R)], [_rand((N, K), 33 + r, dt) for r in range(R)]
+    c = [torch.empty((M, N), dtype=dt, device="cuda") for _ in range(R)]
+    gemm_ar_rd_emulated(ctxs, a, b, c)
+    torch.cuda.synchronize()
+    w.check()
+    assert len(made) == 4        # (256-row panels, which one rank alone would cut from 256-wide pair tiles)
+    assert all(d["bn"] == 128 and not d["by_rounds"] and not d["early_start"] for d in made)
+    ref = sum(a[s].float() @ b[s].float().t() for s in range(R))
+    assert all((x.float() - ref).abs().max().item() < 2e-2 for x in c)
+
+
 def test_gemm_ar_rd_ack_wait_runs_out():
     """A staging slot whose previous occupant is never acknowledged: the exchange kernel's wait
     runs out (20 ms limit), the kernel returns with a status record naming the ack ticket, the

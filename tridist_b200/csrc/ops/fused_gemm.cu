@@ -71,6 +71,7 @@ struct GemmPlan {
   int cta_m;
   int cta_mt;
   int grid_x;
+  bool early_start;
   GemmParams* dev_params = nullptr;   // emulated multi-rank launches only
 };
 
@@ -419,6 +420,7 @@ int64_t gemm_plan_create(const GemmPlanDesc& d) {
   auto* plan = new GemmPlan();
   plan->bn = d.bn;
   plan->bf16 = d.bf16;
+  plan->early_start = d.early_start && d.R == 1;
   plan->cta_m = choose_cta_m(d);
   plan->cta_mt = choose_cta_mt(d, plan->cta_m);
   for (int par = 0; par < 2; ++par) {
@@ -602,10 +604,10 @@ std::vector<std::array<int, 7>> gemm_variants() {
 }
 
 template <int BN, bool kBf16, int kCtaM, bool kStaging, int kMT>
-static void launch_one(const GemmParams& p, int grid_x, cudaStream_t stream) {
+static void launch_one(const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   set_attr_once<BN, kBf16, kCtaM, kStaging, kMT>();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid_x, 1, 1);
+  cfg.gridDim = dim3(plan.grid_x, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = TileShape<BN, kCtaM, kStaging, kMT>::kSmemBytes;
   cfg.stream = stream;
@@ -616,7 +618,7 @@ static void launch_one(const GemmParams& p, int grid_x, cudaStream_t stream) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (p.R == 1 && p.order_table == nullptr) {
+  if (plan.early_start && p.order_table == nullptr) {
     // (an order table, which the kernel before may have written, is read ahead of griddep_wait)
     // Local launches follow one another without a gap: barriers, tensor memory and descriptors
     // of this one are set up while the previous kernel of the stream drains. (Launches that wait
@@ -646,18 +648,18 @@ void gemm_plan_launch(int64_t id, uint32_t round, int parity, int64_t order_tabl
 #define TDB_LAUNCH(BN_, PAIR_)                                                              \
   do {                                                                                      \
     if (plan->bf16) {                                                                       \
-      if (staging) launch_one<BN_, true, PAIR_, true, 1>(p, plan->grid_x, stream);          \
-      else launch_one<BN_, true, PAIR_, false, 1>(p, plan->grid_x, stream);                 \
+      if (staging) launch_one<BN_, true, PAIR_, true, 1>(p, *plan, stream);          \
+      else launch_one<BN_, true, PAIR_, false, 1>(p, *plan, stream);                 \
     } else {                                                                                \
-      if (staging) launch_one<BN_, false, PAIR_, true, 1>(p, plan->grid_x, stream);         \
-      else launch_one<BN_, false, PAIR_, false, 1>(p, plan->grid_x, stream);                \
+      if (staging) launch_one<BN_, false, PAIR_, true, 1>(p, *plan, stream);         \
+      else launch_one<BN_, false, PAIR_, false, 1>(p, *plan, stream);                \
     }                                                                                       \
   } while (0)
   if (plan->bn == 256) {
     if (plan->cta_m == 2 && plan->cta_mt == 2) {
       // 256 rows per CTA: the ring has four stages and the staging area is always there
-      if (plan->bf16) launch_one<256, true, 2, true, 2>(p, plan->grid_x, stream);
-      else launch_one<256, false, 2, true, 2>(p, plan->grid_x, stream);
+      if (plan->bf16) launch_one<256, true, 2, true, 2>(p, *plan, stream);
+      else launch_one<256, false, 2, true, 2>(p, *plan, stream);
     } else if (plan->cta_m == 2) {
       TDB_LAUNCH(256, 2);
     } else {

@@ -256,14 +256,16 @@ def plain_world():
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None,
-            bn: Optional[int] = None, swiglu: bool = False, max_ctas: int = 0, probe: int = 0) -> torch.Tensor:
+            bn: Optional[int] = None, swiglu: bool = False, max_ctas: int = 0, probe: int = 0,
+            local: bool = True) -> torch.Tensor:
     """``out = a @ b.T`` on the hand-written tcgen05 kernel (fp32 accumulate).
 
     With ``swiglu=True`` b holds ``[gate; up]`` row blocks (2*I rows) and the
     result is ``silu(a @ gate.T) * (a @ up.T)`` of shape [M, I], computed in the
     GEMM epilogue. ``probe`` = 1 / 2 runs the pipeline probes (tensor-pipe ceiling: resident
     stages re-multiplied without loads; operand-feed ceiling: loads without MMAs); the output
-    is then meaningless.
+    is then meaningless. ``local=False``: the GEMM is a step of an operator of several ranks, which
+    keeps the tiles and the plain stream order its exchange was measured with.
     """
     assert a.is_cuda and b.is_cuda and a.dtype == b.dtype
     M, K = a.shape
@@ -273,10 +275,10 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     assert out.stride(1) == 1
     if bn is None:
-        bn = choose_bn(M, N, swiglu, K=K, local=True)
+        bn = choose_bn(M, N, swiglu, K=K, local=local and not max_ctas)    # (the rule counts on all SMs)
     w = plain_world()
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-           out.stride(0), bn, swiglu, a.dtype, max_ctas, probe)
+           out.stride(0), bn, swiglu, a.dtype, max_ctas, probe, local)
 
     def make():
         d = base_desc(w, 0, 1, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_PLAIN)
@@ -286,6 +288,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
         if max_ctas:
             d["max_ctas"] = max_ctas
         d["probe"] = probe
+        if not local:
+            d["by_rounds"] = d["early_start"] = 0
         debug_check(d, c_bytes=tensor_extent_bytes(out))
         return native().gemm_plan_create(d)
 

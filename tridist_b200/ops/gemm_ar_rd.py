@@ -172,7 +172,7 @@ def gemm_ar_rd_op(a, b, c, ctx, component="full"):
         r0 = i * CR
         rows = min(CR, M - r0)
         c_panel = c[r0:r0 + rows]
-        gemm_nt(a[r0:r0 + rows], b, out=c_panel, max_ctas=max_ctas)
+        gemm_nt(a[r0:r0 + rows], b, out=c_panel, max_ctas=max_ctas, local=False)
         if not full:
             continue
         slot = i % S
@@ -213,7 +213,7 @@ def gemm_ar_rd_emulated(ctxs, a_list, b_list, c_list):
         blocks = []
         for ctx, a, b, c, base in zip(ctxs, a_list, b_list, c_list, bases):
             c_panel = c[r0:r0 + rows]
-            gemm_nt(a[r0:r0 + rows], b, out=c_panel)
+            gemm_nt(a[r0:r0 + rows], b, out=c_panel, local=False)
             slot = i % S
             ticket = base + i + 1
             prev, ctx.rd.last_ticket_per_slot[slot] = ctx.rd.last_ticket_per_slot[slot], ticket

@@ -50,7 +50,7 @@ def gemm_rs_v5_op(a, b, out, ctx, component="full"):
     if component == "gemm":
         m_pr = a.shape[0] // ctx.num_ranks
         if a.is_cuda:
-            gemm_nt(a[ctx.rank * m_pr:(ctx.rank + 1) * m_pr], b, out=out)
+            gemm_nt(a[ctx.rank * m_pr:(ctx.rank + 1) * m_pr], b, out=out, local=ctx.num_ranks == 1)
         else:
             out.copy_((a[ctx.rank * m_pr:(ctx.rank + 1) * m_pr].float() @ b.float().t()).to(out.dtype))
         return out
