@@ -881,6 +881,56 @@ def test_moe_round_of_any_size(T, E, H, topk, dt):
     finalize_moe_a2a_context(ctx)
 
 
+@pytest.mark.parametrize("T,E,H,topk,dt", [
+    (592, 16, 4096, 6, torch.bfloat16),        # ring: fewest tokens, stages of six rows
+    (600, 32, 8192, 20, torch.float16),        # two runs of a row, a last group of four rows
+    (700, 16, 4096, 5, torch.float16),         # by registers: a ring stage would be too empty
+    (480, 16, 4104, 3, torch.bfloat16),        # four pieces per lane, the last run one piece wide
+    (300, 64, 4096, 17, torch.float16),        # two pieces per lane, five groups of four rows
+    (2500, 8, 512, 2, torch.bfloat16),
+    (3000, 8, 1016, 1, torch.float16),
+])
+def test_moe_combine_by_ring_and_by_registers(T, E, H, topk, dt):
+    test_moe_round_of_any_size(T, E, H, topk, dt)
+
+
+@pytest.mark.parametrize("T,H,topk", [(9, 264, 3), (600, 4096, 6)])
+def test_moe_combine_of_infinities_and_dropped_pairs(T, H, topk):
+    """Both forms: an expert's infinity or NaN reaches the token, a pair without a row adds weight times zero
+    (a NaN where that weight is infinite), and other tokens are untouched."""
+    from tridist_b200.ops import (create_moe_a2a_intra_node_context, finalize_moe_a2a_context,
+                                  moe_combine_intra_node_op, moe_dispatch_intra_node_op)
+    E, dt = 16, torch.bfloat16
+    w = _world1()
+    ctx = create_moe_a2a_intra_node_context(E, H, dt, T, topk, 0, 1, BLOCK_H=H, world=w)
+    tokens = _rand((T, H), 5, dt, scale=1.0)
+    idx = torch.stack([torch.arange(topk, device="cuda") + t % (E - topk) for t in range(T)]).to(torch.int32)
+    idx[4, 1] = -1
+    idx[6, 2] = E
+    wts = torch.rand((T, topk), device="cuda") + 0.5
+    wts[6, 2] = float("inf")
+    wts[7, 0] = 0.0
+    moe_dispatch_intra_node_op(tokens, idx, ctx)
+    sc = ctx.scatter_idx[:T].long()
+    ctx.out[:T * topk] = ctx.recv[:T * topk]
+    ctx.out[sc[2, 1], 7] = float("inf")
+    ctx.out[sc[7, 0], 8] = float("inf")          # times a weight of zero
+    ctx.out[sc[8, 2], H - 1] = float("nan")
+    rows = torch.where((sc >= 0).unsqueeze(2), ctx.out[sc.clamp(min=0)].double(), 0.0)
+    exact = (rows * wts.double().unsqueeze(2)).sum(1)
+    out = torch.empty_like(tokens)
+    moe_combine_intra_node_op(ctx, idx, out, wts)
+    torch.cuda.synchronize()
+    w.check()
+    bad = ~torch.isfinite(exact)
+    assert int(bad.sum()) == H + 3 and torch.equal(torch.isnan(out), torch.isnan(exact))
+    assert torch.equal(out[torch.isinf(exact)].double(), exact[torch.isinf(exact)])
+    # one rounding to bf16 (2^-8) after topk fp32 sums of values up to 2^3 or so
+    diff = (out.double() - exact)[~bad].abs()
+    assert bool((diff <= exact[~bad].abs() * 2.0 ** -8 + 2 * topk * 2.0 ** -24 * 16).all())
+    finalize_moe_a2a_context(ctx)
+
+
 def _gemm_bound(a, b, exact, dt):
     """Largest error of one rounding to 16 bits (half an ulp: 2^-11 of fp16's 11-bit, 2^-8 of bf16's 8-bit
     significand) after an fp32 sum of K products in any order."""

@@ -264,14 +264,19 @@ moe_dispatch_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restric
 }
 
 // ----------------------------------------------------------------------------
-// Combine: pull model, bound by the reads of topk expert rows per token. A CTA works through its
-// (token, run of kRunBytes) units with a ring of stages in shared memory: lane j of the producer
-// warp looks the token's j-th row up (one item ahead) and copies its run into the stage with one
-// bulk copy, so a whole 8 KB row is one request and 192 KB per SM are in flight whatever the
-// look-ups take. Warp w sums its 16-byte columns of the stage, in fp32 and in the order of j.
-// 20 011 tokens of 8 KB rows, topk 8: 412 us with loads into registers, 363 us with 1 KB copies
-// by each warp (as much in flight: scattered 1 KB reads are what DRAM serves slowly), 237 us with
-// whole rows, 6.2 TB/s. 4096 tokens: 68, 79 and 58 us.
+// Combine: pull model, bound by the reads of topk expert rows per token. fp32 sums in the order of a
+// token's experts, in two forms with the same bits.
+//
+// By registers (moe_combine_rows_kernel): one warp per (token, run of 32 * V 16-byte pieces), lane j
+// looking the token's j-th row up one unit ahead, eight loads per lane on their way at a time. As many
+// bytes in flight for one expert per token or a narrow row as for many and a wide one.
+//
+// By a ring (moe_combine_kernel): a CTA works through its (token, 8 KB run) units with three stages of
+// eight rows in shared memory. Lane j of the producer warp looks the token's j-th row up (one item ahead)
+// and copies its run into the stage with one bulk copy; warp w sums its 16-byte columns of the stage.
+// A whole 8 KB row is one request and a full stage keeps 64 KB in flight whatever the look-ups take,
+// where scattered reads of 2 KB are what DRAM serves slowly: 20 011 tokens of 8 KB rows, topk 8, 237 us,
+// 6.2 TB/s. A stage that is not full is wasted: 24 KB in flight at topk 1 (see launch_combine).
 // ----------------------------------------------------------------------------
 template <bool kBf16>
 __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& v, float w) {
@@ -303,23 +308,108 @@ __device__ __forceinline__ uint4 pack8(const float (&a)[8]) {
   return o;
 }
 
-constexpr int kCombineWarps = 8;        // and one more that produces
-constexpr int kCombineRows = 8;         // expert rows per stage
+// "My expert outputs are complete" to every rank, and the same from every rank. False = gave up (all
+// threads of the CTA agree).
+__device__ __forceinline__ bool combine_ready(const MoeDesc& d, int cta, int tid) {
+  if (cta == 0 && tid < d.R) {
+    __threadfence_system();
+    st_release_sys(d.peer_ready_flags[tid] + d.rank, d.round);
+  }
+  int ok = 1;
+  if (tid < d.R)
+    ok = wait_flag_ge(d.peer_ready_flags[d.rank] + tid, d.round, d.env, SITE_MOE_COMBINE_READY, tid) ? 1 : 0;
+  return __syncthreads_and(ok) != 0;
+}
 
-template <int V>
-struct CombineShape {
-  static constexpr int kRunBytes = kCombineWarps * 32 * V * 16;
-  static constexpr int kStageBytes = kCombineRows * kRunBytes;
-  static constexpr int kDepth = 192 * 1024 / kStageBytes;
-  static constexpr int kRingBytes = kDepth * kStageBytes;
-};
+// First byte of the expert row of a pair, or nullptr where it has none (an expert that does not exist, a
+// pair dropped at dispatch, a row out of range, which is recorded when `report` is set).
+__device__ __forceinline__ const uint8_t* expert_row(const MoeDesc& d, int e, int row, int64_t row_bytes, bool report) {
+  if (e < 0 || e >= d.E) return nullptr;
+  if (row >= 0 && row < d.max_recv_rows) return reinterpret_cast<const uint8_t*>(d.peer_out[e / d.epr]) + row * row_bytes;
+  if (row != -1 && report)
+    report_failure(d.env, ST_BAD_INDEX, SITE_INDEX_CHECK, static_cast<uint32_t>(d.max_recv_rows),
+                   static_cast<uint32_t>(row), e);
+  return nullptr;
+}
 
 template <bool kBf16, int V>
+__global__ void __launch_bounds__(kRowThreads)
+moe_combine_rows_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict__ dv, int nv) {
+  TDB_MOE_PROLOGUE
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  griddep_wait();
+  if (d.R == 1) griddep_launch();
+  if (d.R > 1 && !combine_ready(d, cta, tid)) return;
+  constexpr int kRows = 8 / V;            // expert rows whose pieces are loaded together
+  const int64_t row_bytes = static_cast<int64_t>(d.H) * 2;
+  const int n16 = static_cast<int>(row_bytes >> 4);
+  const int runs = (n16 + 32 * V - 1) / (32 * V);
+  const int topk = d.topk;
+  const int64_t units = static_cast<int64_t>(d.T) * runs;
+  const int64_t step = static_cast<int64_t>(ncta) * (kRowThreads / 32);
+  int64_t unit = static_cast<int64_t>(cta) * (kRowThreads / 32) + warp;
+  int e = -1, row = -1;
+  float w = 0.f;
+  auto look_up = [&](int64_t n) {
+    if (n < units && lane < topk) {
+      const int64_t pair = n / runs * topk + lane;
+      e = d.topk_idx[pair];
+      row = d.scatter_idx[pair];
+      w = d.has_weights ? d.topk_weights[pair] : 1.0f;
+    }
+  };
+  look_up(unit);
+  for (; unit < units; unit += step) {
+    const int64_t t = unit / runs;
+    const int run = static_cast<int>(unit - t * runs);
+    const int i0 = run * 32 * V + lane;
+    const uint8_t* src = lane < topk ? expert_row(d, e, row, row_bytes, run == 0) : nullptr;
+    const float my_w = w;
+    look_up(unit + step);
+    float acc[V][8];
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[u][q] = 0.f;
+#pragma unroll 1
+    for (int j0 = 0; j0 < topk; j0 += kRows) {
+      uint4 v[kRows][V];
+#pragma unroll
+      for (int b = 0; b < kRows; ++b) {
+        const uint8_t* from = reinterpret_cast<const uint8_t*>(
+            __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(src), (j0 + b) & 31));
+        const bool have = j0 + b < topk && from != nullptr;
+#pragma unroll
+        for (int u = 0; u < V; ++u)
+          v[b][u] = (have && i0 + 32 * u < n16) ? ld_global_cg_v4(from + (static_cast<int64_t>(i0 + 32 * u) << 4))
+                                                : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int b = 0; b < kRows; ++b) {
+        const float wj = __shfl_sync(0xFFFFFFFFu, my_w, (j0 + b) & 31);
+        if (j0 + b < topk) {
+#pragma unroll
+          for (int u = 0; u < V; ++u) fma8<kBf16>(acc[u], v[b][u], wj);
+        }
+      }
+    }
+    uint8_t* dst = reinterpret_cast<uint8_t*>(d.output) + t * row_bytes;
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+      if (i0 + 32 * u < n16) st_global_v4(dst + (static_cast<int64_t>(i0 + 32 * u) << 4), pack8<kBf16>(acc[u]));
+  }
+}
+
+constexpr int kCombineWarps = 8;        // and one more that produces
+constexpr int kCombineRows = 8;         // expert rows per stage
+constexpr int kRunBytes = 8192;         // of a row, per stage
+constexpr int kStageBytes = kCombineRows * kRunBytes;
+constexpr int kDepth = 3;               // stages (192 KB)
+
+template <bool kBf16>
 __global__ void __launch_bounds__((kCombineWarps + 1) * 32)
 moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict__ dv, int nv) {
   TDB_MOE_PROLOGUE
-  using CS = CombineShape<V>;
-  constexpr int kDepth = CS::kDepth;
   extern __shared__ __align__(128) uint8_t ring[];
   __shared__ __align__(8) uint64_t s_full[kDepth], s_empty[kDepth];
   __shared__ float s_w[kDepth][kCombineRows];
@@ -334,19 +424,12 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
   griddep_wait();
   if (d.R == 1) griddep_launch();
   if (d.R > 1) {
-    if (cta == 0 && tid < d.R) {
-      __threadfence_system();
-      st_release_sys(d.peer_ready_flags[tid] + d.rank, d.round);
-    }
-    int ok = 1;
-    if (tid < d.R)
-      ok = wait_flag_ge(d.peer_ready_flags[d.rank] + tid, d.round, d.env, SITE_MOE_COMBINE_READY, tid) ? 1 : 0;
-    if (!__syncthreads_and(ok)) return;
+    if (!combine_ready(d, cta, tid)) return;
     fence_proxy_async_all();        // what the peers' kernels stored, before the bulk copies read it
   }
 
   const int64_t row_bytes = static_cast<int64_t>(d.H) * 2;
-  const int runs = static_cast<int>((row_bytes + CS::kRunBytes - 1) / CS::kRunBytes);
+  const int runs = static_cast<int>(row_bytes / kRunBytes);      // (the launch asks for whole runs)
   const int topk = d.topk;
   const int groups = (topk + kCombineRows - 1) / kCombineRows;
   const int64_t units = static_cast<int64_t>(d.T) * runs;
@@ -386,24 +469,16 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
           wait_mbar(&s_full[s], s < slot ? phase : phase ^ 1u, quiet, SITE_PIPE_FULL, s);
         return;
       }
-      const uint8_t* src = nullptr;
-      if (e >= 0 && e < d.E) {
-        if (row >= 0 && row < d.max_recv_rows)
-          src = reinterpret_cast<const uint8_t*>(d.peer_out[e / d.epr]) + row * row_bytes;
-        else if (row != -1 && run == 0)                                  // -1 = dropped at dispatch
-          report_failure(d.env, ST_BAD_INDEX, SITE_INDEX_CHECK, static_cast<uint32_t>(d.max_recv_rows),
-                         static_cast<uint32_t>(row), e);
-      }
-      const int64_t off = static_cast<int64_t>(run) * CS::kRunBytes;
-      const uint32_t bytes = static_cast<uint32_t>(min(static_cast<int64_t>(CS::kRunBytes), row_bytes - off));
+      const uint8_t* src = expert_row(d, e, row, row_bytes, run == 0);
+      const int64_t off = static_cast<int64_t>(run) * kRunBytes;
       const uint32_t have = __ballot_sync(0xFFFFFFFFu, src != nullptr);
       if (lane < kCombineRows) s_w[slot][lane] = w;
       if (lane == 0) s_have[slot] = have;
       __syncwarp();                     // the weights before the arrival that publishes the stage
-      if (lane == 0) mbar_arrive_expect_tx(&s_full[slot], bytes * __popc(have));
+      if (lane == 0) mbar_arrive_expect_tx(&s_full[slot], kRunBytes * __popc(have));
       __syncwarp();
       if (src != nullptr)
-        bulk_load_1d(ring + slot * CS::kStageBytes + lane * CS::kRunBytes, src + off, bytes, &s_full[slot]);
+        bulk_load_1d(ring + slot * kStageBytes + lane * kRunBytes, src + off, kRunBytes, &s_full[slot]);
       if (++slot == kDepth) { slot = 0; phase ^= 1u; }
       if (++group == groups) { group = 0; unit += ncta; }
       if (k + 1 < items) look_up();
@@ -411,8 +486,9 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
     return;
   }
 
-  const int col = (warp * 32 + lane) * 16;          // first of this lane's V columns of the run
+  constexpr int V = kRunBytes / (kCombineWarps * 512);      // 16-byte columns per lane
   constexpr int kColStep = kCombineWarps * 512;
+  const int col = (warp * 32 + lane) * 16;                  // the first of them
   float acc[V][8];
   int64_t unit = cta;
   int group = 0;
@@ -429,14 +505,14 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
     if (!ok) return;
     const uint32_t have = s_have[slot];
     const int rows = min(kCombineRows, topk - group * kCombineRows);
-    const uint8_t* stage = ring + slot * CS::kStageBytes + col;
+    const uint8_t* stage = ring + slot * kStageBytes + col;
 #pragma unroll
     for (int j = 0; j < kCombineRows; ++j) {
       if (j >= rows) break;
       const float w = s_w[slot][j];
 #pragma unroll
       for (int u = 0; u < V; ++u) {
-        const uint4 v = (have >> j & 1u) ? *reinterpret_cast<const uint4*>(stage + j * CS::kRunBytes + u * kColStep)
+        const uint4 v = (have >> j & 1u) ? *reinterpret_cast<const uint4*>(stage + j * kRunBytes + u * kColStep)
                                          : make_uint4(0u, 0u, 0u, 0u);
         fma8<kBf16>(acc[u], v, w);
       }
@@ -446,12 +522,10 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
     if (++slot == kDepth) { slot = 0; phase ^= 1u; }
     if (++group == groups) {
       const int t = static_cast<int>(unit / runs);
-      const int64_t off = (unit - static_cast<int64_t>(t) * runs) * CS::kRunBytes + col;
+      const int64_t off = (unit - static_cast<int64_t>(t) * runs) * kRunBytes + col;
 #pragma unroll
       for (int u = 0; u < V; ++u)
-        if (off + u * kColStep < row_bytes)
-          st_global_v4(reinterpret_cast<uint8_t*>(d.output) + t * row_bytes + off + u * kColStep,
-                       pack8<kBf16>(acc[u]));
+        st_global_v4(reinterpret_cast<uint8_t*>(d.output) + t * row_bytes + off + u * kColStep, pack8<kBf16>(acc[u]));
       group = 0;
       unit += ncta;
     }
@@ -534,31 +608,40 @@ static void launch_dispatch(const MoeDesc& d, const MoeDesc* dev, int nv, cudaSt
   else launch(moe_dispatch_kernel<1>, g, kRowThreads, 0, d, dev, nv, s);
 }
 
-template <bool kBf16, int V>
-static void launch_combine_v(const MoeDesc& d, const MoeDesc* dev, int nv, cudaStream_t s) {
-  auto* kernel = moe_combine_kernel<kBf16, V>;
+template <bool kBf16>
+static void launch_combine_ring(const MoeDesc& d, const MoeDesc* dev, int nv, cudaStream_t s) {
+  auto* kernel = moe_combine_kernel<kBf16>;
   static std::atomic<uint64_t> ready{0};      // devices on which the ring's size has been allowed
   int dev_id = 0;
   check(cudaGetDevice(&dev_id), "cudaGetDevice");
   if (!(ready.load() >> (dev_id & 63) & 1u)) {
-    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CombineShape<V>::kRingBytes),
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDepth * kStageBytes),
           "cudaFuncSetAttribute(combine ring)");
     ready.fetch_or(1ull << (dev_id & 63));
   }
-  const int64_t row_bytes = static_cast<int64_t>(d.H) * 2;
-  const int64_t runs = (row_bytes + CombineShape<V>::kRunBytes - 1) / CombineShape<V>::kRunBytes;
-  int64_t g = static_cast<int64_t>(d.T) * runs;
-  if (g > 148) g = 148;
-  if (g < 1) g = 1;
-  launch(kernel, static_cast<int>(g) * nv, (kCombineWarps + 1) * 32, CombineShape<V>::kRingBytes, d, dev, nv, s);
+  launch(kernel, 148 * nv, (kCombineWarps + 1) * 32, kDepth * kStageBytes, d, dev, nv, s);
+}
+
+template <bool kBf16, int V>
+static void launch_combine_rows(const MoeDesc& d, const MoeDesc* dev, int nv, cudaStream_t s) {
+  launch(moe_combine_rows_kernel<kBf16, V>, row_ctas(d, V, 16) * nv, kRowThreads, 0, d, dev, nv, s);
 }
 
 template <bool kBf16>
 static void launch_combine(const MoeDesc& d, const MoeDesc* dev, int nv, cudaStream_t s) {
-  // whole 8 KB rows where every SM has a few tokens; 4 KB runs for narrower rows and, so that twice
-  // as many SMs take part, for few tokens (64 tokens of 8 KB: 128 CTAs, 4.5 us)
-  if (d.H >= 4096 && d.T >= 148 * 4) launch_combine_v<kBf16, 2>(d, dev, nv, s);
-  else launch_combine_v<kBf16, 1>(d, dev, nv, s);
+  // The ring where its stages fill: whole 8 KB runs, six of the eight rows, a few tokens for every SM.
+  // 32768 tokens, us by ring and by registers: 8 KB rows, topk 8 395 and 434, topk 6 336 and 346, topk 4
+  // 295 and 254, topk 1 238 and 123; 2 KB rows, topk 8 320 and 125; 4096 tokens of 10 KB rows, topk 8 96 and
+  // 86, of 8 KB rows, topk 16 109 and 117; 512 tokens of 8 KB rows, topk 8 20 and 18.
+  const int groups = (d.topk + kCombineRows - 1) / kCombineRows;
+  if ((d.H * 2) % kRunBytes == 0 && 4 * d.topk >= 3 * kCombineRows * groups && d.T >= 148 * 4) {
+    launch_combine_ring<kBf16>(d, dev, nv, s);
+    return;
+  }
+  const int v = row_pieces(d, 4);
+  if (v == 4) launch_combine_rows<kBf16, 4>(d, dev, nv, s);
+  else if (v == 2) launch_combine_rows<kBf16, 2>(d, dev, nv, s);
+  else launch_combine_rows<kBf16, 1>(d, dev, nv, s);
 }
 
 void moe_meta_launch(const MoeDesc& d, void* stream_) {
