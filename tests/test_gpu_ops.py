@@ -966,6 +966,24 @@ def test_split_tiles_are_summed_by_their_workers(M, N, K, bn, swiglu):
             assert bool(((out.double() - exact).abs() <= _gemm_bound(a, b, exact, dt)).all())
 
 
+@pytest.mark.parametrize("N,K", [(1024, 4096), (2304, 4096)])      # eight and four slices
+def test_split_tiles_have_the_bits_of_a_sum_by_one_worker(N, K):
+    """A tile summed by all its workers against the same tiles summed by slice 0: a one-shot all-reduce of two
+    virtual ranks, the second with zeros, on as many CTAs per rank."""
+    from tridist_b200.ops._gemm_common import gemm_nt
+    from tridist_b200.ops.gemm_allreduce import create_gemm_ar_intra_node_context, gemm_ar_emulated
+    R, M, dt = 2, 128, torch.bfloat16
+    w = _emu(R)
+    ctxs = [create_gemm_ar_intra_node_context(M, N, dt, dt, r, R, M_PER_CHUNK=64, world=w) for r in range(R)]
+    a, b = _rand((M, K), 91, dt), _rand((N, K), 92, dt)
+    c = [torch.empty((M, N), dtype=dt, device="cuda") for _ in range(R)]
+    gemm_ar_emulated(ctxs, [a, torch.zeros_like(a)], [b, b], c, mode="one_shot")
+    out = gemm_nt(a, b, bn=128, max_ctas=74)
+    torch.cuda.synchronize()
+    w.check()
+    assert torch.equal(out, c[0])
+
+
 def test_split_k_on_several_streams_and_under_capture():
     """Launches that overlap on different streams do not share scratch; a capture on a stream that has not been used before works (what its replays
     compute with new inputs: test_captured_split_k_sums_the_partials_of_its_own_replay)."""

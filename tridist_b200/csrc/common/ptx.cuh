@@ -167,6 +167,14 @@ __device__ __forceinline__ uint4 ld_global_cg_v4(const void* p) {
                : "l"(p));
   return v;
 }
+// Generic address: shared memory, or global memory that bypasses L1.
+__device__ __forceinline__ uint4 ld_cg_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.cg.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint4 ld_global_nc_v4(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"

@@ -586,16 +586,17 @@ __device__ __forceinline__ void split_leave(const GemmParams& p, int slot_s0, in
 
 // Epilogue of a worker's K range of a cut tile (all four epilogue warps). Where the tile goes to other
 // ranks (`local` false) slices 1 .. slices-1 park their accumulator here, for slice 0 to add. Where it
-// stays on this GPU every slice parks the columns that it does not sum itself, waits for the others'
-// and stores the sum of its share: one worker adding all the partials would read slices - 1 whole
-// accumulators through one SM (128 tokens against 7168 x 8192 and 8192 x 3584 weights, five and two
-// slices: 80 us that way, 68 us shared). Scratch layout of a slot: [accumulator block][32-column chunk]
-// [16-byte piece][thread]. Called behind the tile loop: a call inside it kept the loop's state live
-// across this and made every variant of the kernel spill (400 to 1300 bytes of loads).
+// stays on this GPU every slice keeps its share of the columns in shared memory, parks the others',
+// waits for theirs and stores the sum of its share: one worker adding all the partials would read
+// slices - 1 whole accumulators through one SM (128 tokens against 7168 x 8192 and 8192 x 3584 weights,
+// five and two slices: 80 us that way, 68 us shared). Scratch layout of a slot: [accumulator block]
+// [32-column chunk][16-byte piece][thread]. Called behind the tile loop: a call inside it kept the
+// loop's state live across this and made every variant of the kernel spill (400 to 1300 bytes of loads).
 template <int BN, bool kBf16, int kCtaM, int kMT>
 __device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int slice, int slices, int m_tile, int n_tile,
-                                              uint32_t tmem_base, uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar,
-                                              volatile int32_t* s_flags, int it, int my_worker, int sub) {
+                                           uint8_t* ring, uint32_t tmem_base, uint64_t* tmem_full_bar,
+                                           uint64_t* tmem_empty_bar, volatile int32_t* s_flags, int it, int my_worker,
+                                           int sub) {
   const WaitEnv& env = p.env;
   const int lane = threadIdx.x & 31;
   const int q = (threadIdx.x >> 5) & 3;                // TMEM lane quarter this warp may read
@@ -622,6 +623,11 @@ __device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int 
   const int u_hi = units * (slice + 1) / slices;
   const uint32_t tq = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
                       static_cast<uint32_t>((kMT == 2) ? 0 : (it & 1) * BN);
+  // The sum is in the order of the slices whichever of them adds (the bits of a sum by slice 0). Slices 0
+  // and 1 can start from their own columns in tensor memory (a + b is b + a); the others keep theirs in
+  // shared memory and add them when it is their turn.
+  const bool first = slice < 2;
+  const int halves = swiglu ? 2 : 1;
   auto release = [&]() {
     tc_fence_before_sync();
     __syncwarp();
@@ -633,14 +639,27 @@ __device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int 
       }
     }
   };
+  constexpr int kChunkBytes = 32 * 4 * kEpiThreads;
   float* const dst = p.sk_ws + static_cast<int64_t>(my_slot) * p.sk_slot_words + etid * 4;
+  uint8_t* const own = ring + etid * 16;      // (at most half a tile; the MMAs have read the ring)
 #pragma unroll 1
   for (int hc = 0; hc < kMT * (BN / 32); ++hc) {
-    const int u = swiglu ? hc % (BN / 64) : hc % (BN / 32);
-    if (local && u >= u_lo && u < u_hi) continue;
+    const int h = hc / (BN / 32), c = hc % (BN / 32);
+    const int u = swiglu ? c % (BN / 64) : c;
+    const bool mine = local && u >= u_lo && u < u_hi;
+    if (mine && first) continue;
     uint32_t r[32];
     tmem_ld_32x32b_x32(tq + hc * 32, r);      // (accumulator block 1 follows block 0)
     tmem_ld_wait();
+    if (mine) {
+      // in the order of use: block, share unit, (gate, up)
+      uint8_t* keep = own + ((h * (u_hi - u_lo) + u - u_lo) * halves + (swiglu ? c / (BN / 64) : 0)) * kChunkBytes;
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        *reinterpret_cast<uint4*>(keep + v * (kEpiThreads * 16)) =
+            make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+      continue;
+    }
 #pragma unroll
     for (int v = 0; v < 8; ++v)
       st_global_v4(dst + (hc * 8 + v) * (kEpiThreads * 4),
@@ -653,24 +672,26 @@ __device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int 
     release();
     return true;
   }
-  if (etid == 0) {
-    ok = wait_flag_ge(p.sk_words + slot_s0, static_cast<uint32_t>(slices), env, SITE_SPLITK, slice);
-  }
+  if (etid == 0) ok = wait_flag_ge(p.sk_words + slot_s0, static_cast<uint32_t>(slices), env, SITE_SPLITK, slice);
   if (!epi_vote(s_flags, ok)) return false;
-  // The other slices' pieces in the order they are added: block, share unit, (gate, up), slice.
-  // The next eight 16-byte pieces are on their way while the last ones are added.
-  const int more = slices - 1;
-  const int halves = swiglu ? 2 : 1;
+  // The slices' pieces in the order they are added: block, share unit, (gate, up), slice. The next eight
+  // 16-byte pieces are on their way while the last ones are added.
   int fh = u_lo < u_hi ? 0 : kMT, fu = u_lo, fq = 0, fs = 0;
+  const int adds = first ? slices - 1 : slices;
+  const uint8_t* kept = own;
   uint4 nx[8];
   auto fetch = [&]() {
     if (fh >= kMT) return;
-    const int s = fs + (fs >= slice ? 1 : 0);
+    const int s = fs + ((first && fs >= slice) ? 1 : 0);
     const float* src = p.sk_ws + (slot_s0 + s * kCtaM) * static_cast<int64_t>(p.sk_slot_words) +
                        ((fh * (BN / 32) + fu + fq * (BN / 64)) * 8 * kEpiThreads + etid) * 4;
+    if (s == slice) {
+      src = reinterpret_cast<const float*>(kept);
+      kept += kChunkBytes;
+    }
 #pragma unroll
-    for (int v = 0; v < 8; ++v) nx[v] = ld_global_cg_v4(src + v * (kEpiThreads * 4));
-    if (++fs == more) {
+    for (int v = 0; v < 8; ++v) nx[v] = ld_cg_v4(src + v * (kEpiThreads * 4));
+    if (++fs == adds) {
       fs = 0;
       if (++fq == halves) {
         fq = 0;
@@ -678,15 +699,20 @@ __device__ __forceinline__ bool split_tile(const GemmParams& p, bool local, int 
       }
     }
   };
-  // own 32 columns of chunk hc plus the other slices'
+  // the next 32 columns (chunk hc of the tile)
   auto sum_chunk = [&](int hc, float (&acc)[32]) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(tq + hc * 32, r);
-    tmem_ld_wait();
+    if (first) {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(tq + hc * 32, r);
+      tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r[j]);
+      for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+    }
 #pragma unroll 1
-    for (int s = 0; s < more; ++s) {
+    for (int s = 0; s < adds; ++s) {
       uint4 x[8];
 #pragma unroll
       for (int v = 0; v < 8; ++v) x[v] = nx[v];
@@ -734,6 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __restrict__ pv) {
   using TS = TileShape<BN, kCtaM, kStaging, kMT>;
   static_assert(kCtaM == 1 || BN == 256, "CTA pairs are built for 256-wide tiles only");
+  static_assert(kMT * BM * BN * 2 <= TS::kStages * TS::kStageBytes, "a slice keeps up to half its tile in the ring");
   // With pv != nullptr the launch emulates several ranks on one GPU: grid.y
   // indexes the rank and each rank reads its own parameter block.
   const GemmParams& p = pv ? pv[blockIdx.y] : p0;
@@ -1576,8 +1603,9 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
       const TileCoord t = tile_at(p, s_order, wi.pos, sub, bands);
       if (alive && t.valid && (split_local || wi.slice > 0)) {
         const uint64_t t_sk0 = (prof && etid == 0) ? globaltimer_ns() : 0;
-        if (split_tile<BN, kBf16, kCtaM, kMT>(p, split_local, wi.slice, wi.slices, t.m_tile, t.n_tile, tmem_base,
-                                              tmem_full_bar, tmem_empty_bar, s_flags, it, my_worker, sub) &&
+        if (split_tile<BN, kBf16, kCtaM, kMT>(p, split_local, wi.slice, wi.slices, t.m_tile, t.n_tile, ring,
+                                              tmem_base, tmem_full_bar, tmem_empty_bar, s_flags, it, my_worker,
+                                              sub) &&
             prof && etid == 0) {
           prof[PROF_SK_WAIT] += globaltimer_ns() - t_sk0;
           prof[PROF_EPI_TILES] += kMT;
