@@ -189,9 +189,12 @@ def test_own_first_band_major_walk():
     assert len(set(later)) >= 3, "several sources side by side"
 
 
+# (us with tall and with short tiles: 761 and 1073, 914 and 1119, 386 and 503, 107 and 120, 388 and 467, 308 and 337;
+# 74 and 74, 2191 and 2079, 104 and 87, 89 and 69)
 @pytest.mark.parametrize("M,N,K,tall", [(8192, 6144, 12288, True), (8192, 12288, 6144, True), (1024, 8192, 28672, True),
-                                        (1984, 8192, 3696, True), (512, 8192, 8192, False), (2112, 4096, 11008, False),
-                                        (2112, 22016, 4096, False), (1280, 16384, 53248, True), (520, 264, 64, False), (513, 8, 8192, False)])
+                                        (1984, 8192, 3696, True), (4096, 8192, 8192, True), (2112, 22016, 4096, True),
+                                        (512, 8192, 8192, False), (1280, 16384, 53248, False), (1600, 16000, 1568, False),
+                                        (2112, 4096, 4096, False), (520, 264, 64, False), (513, 8, 8192, False)])
 def test_tile_height_by_rounds(M, N, K, tall):
     """Local launches take 512-row or 256-row pair tiles by the rounds they need; every tile once either way."""
     out = _dump(M=M, N=N, K=K, bn=256, by_rounds=1)

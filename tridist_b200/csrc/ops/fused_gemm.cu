@@ -126,11 +126,11 @@ static int slices_for(int left, int g, int k_blocks) {
 }
 
 // Rounds that `tiles` pair tiles take on `g` pairs. Parking and adding the partials of a cut round
-// costs about as much as 40 k-blocks of its tiles (12 us of 256 x 256 tiles, 33 us of 512 x 256).
+// costs about as much as 25 k-blocks of its tiles (fitted together with the ratio below).
 static double pair_rounds(int64_t tiles, int g, int k_blocks) {
   const int left = static_cast<int>(tiles % g);
   const int s = slices_for(left, g, k_blocks);
-  const double last = left == 0 ? 0.0 : s > 1 ? std::min(1.0, 1.0 / s + 40.0 / k_blocks) : 1.0;
+  const double last = left == 0 ? 0.0 : s > 1 ? std::min(1.0, 1.0 / s + 25.0 / k_blocks) : 1.0;
   return static_cast<double>(tiles / g) + last;
 }
 
@@ -144,19 +144,19 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
   if (d.op == OP_RS && d.R > 1 && d.sched != SCHED_SEGMENT) return 1;
   if (d.by_rounds) {
     // Half as tall a tile where that takes fewer rounds, or pads fewer rows, than its operand
-    // traffic costs. A round of 256 x 256 tiles takes 1.03 to 1.3 times half a round of 512 x 256
-    // tiles up to K = 12288 (the more rounds, the closer); at 1.08 all of these come out on the faster side, tall
-    // against short, rows x N x K: 512 x 8192 x 8192 81 and 67 us, 2112 x 4096 x 11008 178 and 171,
-    // 2112 x 22016 x 4096 358 and 338; 1984 x 8192 x 3696 104 and 121, 1024 x 8192 x 28672 338 and
-    // 452, 8192 x 6144 x 12288 991 and 1107, 8192 x 12288 x 6144 1016 and 1062.
+    // traffic costs. A round of 256 x 256 tiles takes 1.31 times half a round of 512 x 256 tiles from
+    // K = 16000 on (1.2 to 1.4, to K = 53248), and less for a short K, 1.24 at 6000 and 1.12 at 1500:
+    // the tall tile's accumulators fill tensor memory, so part of its epilogue is in every round. The line
+    // is fitted to 368 shapes of 512 to 8192 rows: 0.1 % above the faster height on average, four shapes
+    // 1 to 3 % slower than tall tiles alone, which take 3 % more. Tall against short, rows x N x K:
+    // 512 x 8192 x 4096 42 and 36 us, 1600 x 16000 x 1568 104 and 87, 1280 x 16384 x 53248 2191 and 2079;
+    // 4096 x 8192 x 8192 388 and 467, 2112 x 22016 x 4096 308 and 337, 1024 x 8192 x 28672 386 and 503,
+    // 8192 x 12288 x 6144 914 and 1119.
     const int bn_out = (d.epi == EPI_SWIGLU) ? d.bn / 2 : d.bn;
     const int64_t nt = (d.N + bn_out - 1) / bn_out;
     const int kb = (d.K + BK - 1) / BK;
     const int g = std::max(1, (d.max_ctas > 0 ? std::min(d.max_ctas, 148) : 148) / 2);
-    // Past K = 12288 a raster group is one or two row units high, half as tall a unit reads B from
-    // DRAM up to twice as often, and the ratio is 1.34 (K 28672 above) to 1.43 (1280 x 16384 x 53248:
-    // 2136 and 2227 us).
-    const double ratio = kb <= 192 ? 1.08 : 1.45;
+    const double ratio = std::max(1.1, 1.35 - 8.0 / kb);
     if (ratio * pair_rounds((mt + 1) / 2 * nt, g, kb) < 2.0 * pair_rounds((mt + 3) / 4 * nt, g, kb)) return 1;
   }
   return 2;
