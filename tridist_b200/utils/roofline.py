@@ -54,5 +54,6 @@ def gemm_ar_roof(M, N, k_loc, R, two_shot=True):
 
 def moe_roof(T, H, topk, R):
     one_way = T * topk * H * 2 * (R - 1) / max(R, 1)
-    # dispatch then combine: each direction carries the rows once; at R = 1 it is an HBM copy
-    return roof_ms(0.0, 2 * one_way if R > 1 else 0.0, hbm_bytes=4.0 * T * topk * H * 2)
+    # dispatch then combine: each direction carries the rows once. In HBM a token is read and written once,
+    # its topk rows are written for the experts and read back
+    return roof_ms(0.0, 2 * one_way if R > 1 else 0.0, hbm_bytes=(2.0 + 2.0 * topk) * T * H * 2)
