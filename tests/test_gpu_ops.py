@@ -894,6 +894,21 @@ def test_moe_combine_by_ring_and_by_registers(T, E, H, topk, dt):
     test_moe_round_of_any_size(T, E, H, topk, dt)
 
 
+def test_moe_context_scratch_is_one_allocation():
+    """The six tensors that only the MoE kernels use share one allocation, each on a 16-byte boundary; with the
+    five that callers read, a context makes six allocations (eight before the metadata had scratch of its own)."""
+    from tridist_b200.ops import create_moe_a2a_intra_node_context, finalize_moe_a2a_context
+    w = _world1()
+    ctx = create_moe_a2a_intra_node_context(7, 64, torch.float16, 5, 3, 0, 1, BLOCK_H=64, world=w)
+    own = [ctx.counters, ctx.dst_row_base, ctx.done_counter, ctx.meta_counter, ctx.slots, ctx.cta_base]
+    assert len({t.untyped_storage().data_ptr() for t in own}) == 1
+    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * 4) for t in own)
+    assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:])) and all(lo % 16 == 0 for lo, _ in spans)
+    read = [ctx.scatter_idx, ctx.splits, ctx.recv_seg, ctx.recv_counts, ctx.recv_total_t]
+    assert len({t.untyped_storage().data_ptr() for t in own + read}) == 6
+    finalize_moe_a2a_context(ctx)
+
+
 @pytest.mark.parametrize("T,H,topk", [(9, 264, 3), (600, 4096, 6)])
 def test_moe_combine_of_infinities_and_dropped_pairs(T, H, topk):
     """Both forms: an expert's infinity or NaN reaches the token, a pair without a row adds weight times zero

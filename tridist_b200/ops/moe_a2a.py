@@ -17,6 +17,7 @@ rows have landed.
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from typing import List, Optional
 
@@ -80,6 +81,16 @@ class MoEA2AContext:
         return self.out.data_ptr()
 
 
+def _carve(device, *shapes):
+    """Zeroed int32 tensors of these shapes, each on a 16-byte boundary of one allocation."""
+    sizes = [math.prod(s) for s in shapes]
+    starts = [0]
+    for n in sizes:
+        starts.append(starts[-1] + -(-n // 4) * 4)
+    whole = torch.zeros(starts[-1], dtype=torch.int32, device=device)
+    return [whole[o:o + n].view(s) for o, n, s in zip(starts, sizes, shapes)]
+
+
 def create_moe_a2a_intra_node_context(num_experts, hidden, dtype, max_tokens, topk, rank, num_ranks,
                                       mpi=None, comm=None, BLOCK_H=1024, world=None,
                                       max_recv_rows: Optional[int] = None):
@@ -99,21 +110,19 @@ def create_moe_a2a_intra_node_context(num_experts, hidden, dtype, max_tokens, to
                         input_dtype=dtype, row_bytes=hidden * elem, BLOCK_H=BLOCK_H, world=world)
     dev = "cpu" if isinstance(world, CpuWorld) else "cuda"
     ctx.scatter_idx = torch.full((max_tokens, topk), -1, dtype=torch.int32, device=dev)
-    ctx.counters = torch.zeros(num_experts, dtype=torch.int32, device=dev)
     ctx.splits = torch.zeros(num_experts, dtype=torch.int32, device=dev)
-    ctx.dst_row_base = torch.zeros(num_experts, dtype=torch.int32, device=dev)
     ctx.recv_seg = torch.zeros((num_ranks, epr), dtype=torch.int32, device=dev)
     ctx.recv_counts = torch.zeros((num_ranks, epr), dtype=torch.int32, device=dev)
     ctx.recv_total_t = torch.zeros(1, dtype=torch.int32, device=dev)
+    # what only the kernels read and write, cut from one allocation
+    n_meta = 0 if isinstance(world, CpuWorld) else native().MOE_META_CTAS
+    ctx.counters, ctx.dst_row_base, ctx.done_counter, ctx.meta_counter, ctx.slots, ctx.cta_base = _carve(
+        dev, (num_experts,), (num_experts,), (1,), (1,), (max_tokens, topk), (n_meta, num_experts))
     if isinstance(world, CpuWorld):
         ctx.recv = torch.zeros((max_recv_rows, hidden), dtype=dtype)
         ctx.out = torch.zeros((max_recv_rows, hidden), dtype=dtype)
         return ctx
     assert elem == 2, "the MoE kernels move 16-bit rows (fp16 / bf16)"
-    ctx.done_counter = torch.zeros(1, dtype=torch.int32, device=dev)
-    ctx.meta_counter = torch.zeros(1, dtype=torch.int32, device=dev)
-    ctx.slots = torch.empty((max_tokens, topk), dtype=torch.int32, device=dev)
-    ctx.cta_base = torch.empty((native().MOE_META_CTAS, num_experts), dtype=torch.int32, device=dev)
     ctx.recv_buf = world.alloc(max_recv_rows * ctx.row_bytes, rank)
     ctx.out_buf = world.alloc(max_recv_rows * ctx.row_bytes, rank)
     ctx.meta_buf = world.alloc(2 * num_ranks * num_experts * 4, rank)
