@@ -1,0 +1,123 @@
+"""The GEMM for at most 128 rows (csrc/gemm/skinny_gemm.cuh) on one GPU, at the edges of its layout."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(shape, seed, dt):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * 0.1).to(dt)
+
+
+def _bound(a, b, exact, dt):
+    """One rounding to 16 bits after an fp32 sum of K products in any order."""
+    half_ulp = 2.0 ** -11 if dt == torch.float16 else 2.0 ** -8
+    return exact.abs() * half_ulp * 1.01 + a.shape[1] * 2.0 ** -23 * (a.abs().double() @ b.abs().double().t()) + 2.0 ** -24
+
+
+@pytest.mark.parametrize("M,N,K,swiglu,cluster", [
+    (1, 8, 8, False, 1), (16, 264, 136, False, 1), (33, 1000, 64, False, 1),
+    (64, 4096, 1376, False, 1),                # a share of 24 or 32 rows of B, last k-block short
+    (65, 1000, 1024, False, 1), (128, 8192, 3584, False, 1), (128, 1408, 4096, False, 2),
+    (100, 48, 8200, False, 4),                 # three shares, four ranges of K
+    (64, 2048, 16384, False, 4), (128, 4096, 12288, False, 4),
+    (128, 40000, 512, False, 1),               # several shares a CTA
+    (96, 30000, 4096, False, 1), (128, 3584, 2048, True, 1), (100, 1416, 4104, True, 2), (40, 20000, 320, True, 1),
+    (128, 128, 8192, True, 4),
+])
+def test_few_rows(M, N, K, swiglu, cluster):
+    from tridist_b200.ops._gemm_common import gemm_nt
+    from tridist_b200.parallel.runtime import native
+    assert native().skinny_layout(M, N, K, swiglu, 148)["cluster"] == cluster
+    for dt in (torch.float16, torch.bfloat16):
+        wide_a, wide_b = _rand((M, K + 24), 1, dt), _rand((2 * N if swiglu else N, K + 8), 2, dt)
+        a, b = wide_a[:, 8:K + 8], wide_b[:, :K]                # row strides of their own, a on a 16-byte boundary
+        plane = torch.full((M + 2, N + 16), 7.0, dtype=dt, device="cuda")
+        out = plane[1:M + 1, 8:N + 8]
+        gemm_nt(a, b, out=out, swiglu=swiglu)
+        first = out.clone()
+        gemm_nt(a, b, out=out, swiglu=swiglu)
+        torch.cuda.synchronize()
+        assert torch.equal(first, out)
+        edge = plane.clone()
+        edge[1:M + 1, 8:N + 8] = 7.0
+        assert bool((edge == 7.0).all())                        # nothing beside the output was written
+        exact = a.double() @ b.double().t()
+        if swiglu:
+            gate, up = exact[:, :N], exact[:, N:]
+            exact = F.silu(gate) * up
+            # the fp32 sums' errors through silu (its slope is below 1.1), __expf and the fast divide: 2^-20
+            e = K * 2.0 ** -23 * (a.abs().double() @ b.abs().double().t())
+            bound = (exact.abs() * (2.0 ** -11 if dt == torch.float16 else 2.0 ** -8) * 1.01 + exact.abs() * 2.0 ** -18 +
+                     1.1 * e[:, :N] * up.abs() + F.silu(gate).abs() * e[:, N:] + 2.0 ** -24)
+        else:
+            bound = _bound(a, b, exact, dt)
+        assert bool(((out.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 4096, 512), (64, 2048, 8192), (128, 8192, 1024)])
+def test_few_rows_keep_infinities_to_their_rows(M, N, K):
+    from tridist_b200.ops._gemm_common import gemm_nt
+    dt = torch.bfloat16
+    a, b = _rand((M, K), 3, dt), _rand((N, K), 4, dt)
+    a[M // 2, K - 1] = float("inf")
+    b[N - 3, 5] = float("nan")
+    out = gemm_nt(a, b)
+    torch.cuda.synchronize()
+    exact = a.double() @ b.double().t()
+    bad = ~torch.isfinite(exact)
+    assert int(bad.sum()) == M + N - 1 and torch.equal(torch.isfinite(out), ~bad)
+    assert torch.equal(torch.isnan(out), torch.isnan(exact))
+
+
+def test_few_rows_on_streams_and_in_graphs():
+    """Replays over other inputs, on two streams beside eager calls: the bits of the eager call."""
+    from tridist_b200.ops._gemm_common import gemm_nt
+    dt = torch.bfloat16
+    for M, N, K in [(64, 4096, 1376), (128, 8192, 8192)]:
+        b = _rand((N, K), 5, dt)
+        a = [torch.zeros((M, K), dtype=dt, device="cuda") for _ in range(2)]
+        outs = [torch.empty((M, N), dtype=dt, device="cuda") for _ in range(2)]
+        gemm_nt(a[0], b)
+        torch.cuda.synchronize()
+        graphs, streams = [torch.cuda.CUDAGraph() for _ in range(2)], [torch.cuda.Stream() for _ in range(2)]
+        for g, s, x, o in zip(graphs, streams, a, outs):
+            with torch.cuda.graph(g, stream=s):
+                gemm_nt(x, b, out=o)
+                gemm_nt(x, b, out=o)
+        for it in range(10):
+            new = [_rand((M, K), 10 + 2 * it + i, dt) for i in range(2)]
+            ref = [gemm_nt(x, b) for x in new]
+            for x, y, o in zip(a, new, outs):
+                x.copy_(y)
+                o.zero_()
+            torch.cuda.synchronize()
+            for g, s in zip(graphs, streams):
+                with torch.cuda.stream(s):
+                    g.replay()
+            between = gemm_nt(new[0], b)
+            torch.cuda.synchronize()
+            assert torch.equal(between, ref[0]) and all(torch.equal(o, r) for o, r in zip(outs, ref))
+
+
+def test_few_rows_of_a_context_follow_the_kernel_in_front():
+    """Each call reads what the call before it wrote, back to back."""
+    from tridist_b200.ops import create_gemm_ar_intra_node_context, finalize_gemm_ar_context, gemm_ar_intra_node_op
+    from tridist_b200.parallel.runtime import ProcessWorld
+    w = ProcessWorld(0, 1)
+    dt, M, N = torch.bfloat16, 64, 2048
+    ctx = create_gemm_ar_intra_node_context(M, N, dt, dt, 0, 1, M_PER_CHUNK=64, world=w)
+    x = [_rand((M, N), 6, dt), torch.empty((M, N), dtype=dt, device="cuda")]
+    b = (_rand((N, N), 7, dt).float() * (10.0 / N ** 0.5)).to(dt)
+    refs = [x[0].clone()]
+    for _ in range(6):
+        refs.append((refs[-1].double() @ b.double().t()).to(dt))
+    for i in range(6):
+        gemm_ar_intra_node_op(x[i & 1], b, x[~i & 1], ctx)
+    torch.cuda.synchronize()
+    w.check()
+    err = (x[0].double() - refs[6].double()).norm() / refs[6].double().norm()
+    assert err < 6 * 2.0 ** -8
+    finalize_gemm_ar_context(ctx)

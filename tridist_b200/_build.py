@@ -29,6 +29,7 @@ SOURCES = [
     "runtime/vmm_heap.cu",
     "runtime/split_scratch.cpp",
     "ops/fused_gemm.cu",
+    "ops/skinny_gemm.cu",
     "ops/elementwise.cu",
     "ops/moe_a2a.cu",
     "ops/rd_exchange.cu",

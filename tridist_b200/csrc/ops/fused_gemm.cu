@@ -14,6 +14,7 @@
 #include <unordered_map>
 
 #include "../gemm/fused_gemm.cuh"
+#include "skinny_gemm.h"
 
 namespace tdb {
 
@@ -72,6 +73,8 @@ struct GemmPlan {
   int cta_mt;
   int grid_x;
   bool early_start;
+  bool skinny = false;                // few rows: launches go to the kernel of skinny_gemm.cuh
+  SkinnyParams few;
   GemmParams* dev_params = nullptr;   // emulated multi-rank launches only
 };
 
@@ -497,6 +500,17 @@ int64_t gemm_plan_create(const GemmPlanDesc& d) {
     p.env.rank = static_cast<uint32_t>(d.rank);
   }
   plan->grid_x = grid_for(d, plan->prm[0], d.max_ctas, num_sms());
+  if (d.few_rows && d.R == 1 && d.M <= 128 && d.prof == 0 && d.c % 16 == 0 && d.ldc % 8 == 0) {
+    plan->skinny = true;
+    SkinnyParams& f = plan->few;
+    f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, num_sms());
+    if (f.swiglu) f.up_row0 = d.swiglu_up_row0;
+    f.tma_a = make_tmap(reinterpret_cast<void*>(d.a), d.a_rows, d.K, d.lda, d.bf16, f.ar);
+    f.tma_b = make_tmap(reinterpret_cast<void*>(d.b), d.b_rows, d.K, d.ldb, d.bf16, f.wr);
+    f.c = reinterpret_cast<void*>(d.c);
+    f.ldc = d.ldc;
+    f.env = plan->prm[0].env;
+  }
   if (d.check_residency) {
     const int fit = resident_ctas_of(*plan);
     if (plan->grid_x > fit) {
@@ -636,6 +650,11 @@ void gemm_plan_launch(int64_t id, uint32_t round, int parity, int64_t order_tabl
                       void* stream_) {
   GemmPlan* plan = find_plan(id);
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (plan->skinny && order_table == 0 && !((flags >> 1) & 1)) {      // (nothing to compute: the general kernel)
+    skinny_launch(plan->few, plan->early_start, stream);
+    ++g_launches;
+    return;
+  }
   GemmParams p = plan->prm[parity & 1];
   p.round = round;
   p.order_table = reinterpret_cast<const int32_t*>(order_table);

@@ -1,0 +1,142 @@
+#include "skinny_gemm.h"
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <stdexcept>
+#include <string>
+
+#include "../gemm/skinny_gemm.cuh"
+
+namespace tdb {
+
+static void check(cudaError_t e, const char* what) {
+  if (e != cudaSuccess)
+    throw std::runtime_error(std::string("tridist_b200: ") + what + ": " + cudaGetErrorString(e));
+}
+
+static int ceil_div(int a, int b) { return (a + b - 1) / b; }
+static int up_to(int a, int m) { return ceil_div(a, m) * m; }
+
+static EvenRuns even_runs(int total, int n) { return {total / n, total % n}; }
+
+// Everything that follows from a cluster size and the most rows of B in a share.
+static SkinnyParams lay_out(int M, int N, int K, bool swiglu, bool bf16, int sms, int cluster_log2, int most) {
+  SkinnyParams p;
+  std::memset(&p, 0, sizeof(p));
+  const int cluster = 1 << cluster_log2;
+  p.M = M;
+  p.N = N;
+  p.k_blocks = ceil_div(K, 64);
+  p.bf16 = bf16 ? 1 : 0;
+  p.swiglu = swiglu ? 1 : 0;
+  p.up_row0 = N;
+  p.cluster_log2 = cluster_log2;
+  p.range = even_runs(p.k_blocks, cluster);
+  p.groups = N / 8;
+  p.boxes = swiglu ? 2 : 1;
+  const int can_run = std::max(1, cluster <= 2 ? sms / cluster : sms * 7 / 8 / cluster);   // (larger clusters leave SMs out)
+  const int rounds = ceil_div(ceil_div(p.groups, can_run), most / 8 / p.boxes);
+  p.shares = std::min(rounds * can_run, ceil_div(p.groups, 2));
+  p.share = even_runs(p.groups, p.shares);
+  p.workers = std::min(p.shares, can_run);
+  p.ar = up_to(M, 8);
+  p.wr = 8 * (p.share.len + (p.share.more > 0 ? 1 : 0));
+  p.nb = up_to(p.wr, 16);
+  p.mma_n = p.boxes * p.nb;
+  p.own = ceil_div(p.wr / 8, cluster);
+  p.warps = ceil_div(M, 32);
+  const int xbuf = (cluster - 1) * p.boxes * p.own * p.warps * 1024;
+  const int block = (p.ar + p.nb * p.boxes) * 128;
+  p.pad = (128 - p.ar) * 128;
+  const int room = kSkinnySmem - p.pad - xbuf;
+  const int range = p.range.len + (p.range.more > 0 ? 1 : 0);
+  p.kw = 8;
+  while (p.kw > 1 && ((p.kw == 8 ? 2 : 3) * p.kw * block > room || p.kw >= 2 * range)) p.kw /= 2;
+  p.stage_bytes = p.kw * block;
+  p.stages = std::min(kSkinnyMaxStages, room / p.stage_bytes);
+  p.stages = std::max(1, std::min(p.stages, ceil_div(range, p.kw) * ceil_div(p.shares, p.workers)));
+  p.smem_bytes = p.stages * p.stage_bytes + p.pad + xbuf;
+  p.acc_cols = up_to(p.mma_n, 32);
+  const int bufs = p.shares > p.workers ? 2 : 1;
+  // runs of 16 k-blocks or more, four of them over the whole of K
+  while (2 << p.accs_log2 <= 4 / cluster && (bufs * p.acc_cols << (p.accs_log2 + 1)) <= 512 &&
+         (32 << p.accs_log2) <= p.range.len) ++p.accs_log2;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < bufs * p.acc_cols << p.accs_log2) p.tmem_cols *= 2;
+  return p;
+}
+
+SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms) {
+  // The expected time: B from DRAM; what a CTA loads in all, at about 120 GB/s through its L2 port, or its k-blocks,
+  // 130 ns each however small; the two overlap, not wholly. A cluster starts later and exchanges parts, 2.5 us for
+  // two CTAs and 5 for four. us measured with clusters of 1, 2 and 4 (rows x N x K): 128 x 8192 x 28672 89.5, 81.7 and 104;
+  // 128 x 8192 x 3584 15.2, 16.6 and 23.7; 64 x 4096 x 1376 7.6, 8.4 and 9.3; 64 x 2048 x 16384 36.7, 25.7 and 21.3;
+  // 128 x 512 x 8192 23.7, 15.9 and 15.5. 128 x 28672 x 8192 by shares of 104 and of 200 rows 92.7 and 76.8.
+  SkinnyParams best;
+  double best_us = -1;
+  for (int cl2 = 0; 1 << cl2 <= kSkinnyMaxCluster; ++cl2)
+    for (int most = 128; most <= 256; most *= 2) {
+      const SkinnyParams p = lay_out(M, N, K, swiglu, bf16, sms, cl2, most);
+      if (cl2 > 0 && (p.range.len < 2 || p.shares > p.workers)) continue;     // (a cluster meets once)
+      if (best_us >= 0 && p.stages * p.stage_bytes < 120 * 1024) continue;    // (too little in flight)
+      const double rounds = ceil_div(p.shares, p.workers);
+      const double dram = static_cast<double>(N) * p.boxes * K * 2 / 6.3e6;
+      const double cta = rounds * (p.range.len + 1) * std::max((p.ar + p.wr * p.boxes) * 128 / 0.12e6, 0.13);
+      const double us = std::max(dram, cta) + 0.3 * std::min(dram, cta) + (cl2 == 0 ? 0.0 : cl2 == 1 ? 2.5 : 5.0);
+      if (best_us < 0 || us < 0.98 * best_us) {
+        best = p;
+        best_us = us;
+      }
+    }
+  return best;
+}
+
+std::vector<std::array<int, 2>> skinny_shares(const SkinnyParams& p) {
+  std::vector<std::array<int, 2>> out;
+  for (int v = 0; v < p.shares; ++v) out.push_back({p.share.start(v), p.share.start(v + 1)});
+  return out;
+}
+
+template <int kW>
+static void launch(const SkinnyParams& p, bool early_start, cudaStream_t stream) {
+  auto* kernel = skinny_gemm_kernel<kW>;
+  static std::atomic<uint64_t> ready{0};      // devices on which the ring's size has been allowed
+  int dev = 0;
+  check(cudaGetDevice(&dev), "cudaGetDevice");
+  if (!(ready.load() >> (dev & 63) & 1u)) {
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSkinnySmem),
+          "cudaFuncSetAttribute(few-rows GEMM)");
+    ready.fetch_or(1ull << (dev & 63));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.workers << p.cluster_log2, 1, 1);
+  cfg.blockDim = dim3(kSkinnyThreads, 1, 1);
+  cfg.dynamicSmemBytes = p.smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1 << p.cluster_log2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early_start ? 2 : 1;
+  check(cudaLaunchKernelEx(&cfg, kernel, p), "few-rows GEMM launch");
+}
+
+void skinny_launch(const SkinnyParams& p, bool early_start, void* stream_) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  switch (p.kw) {
+    case 1: launch<1>(p, early_start, stream); break;
+    case 2: launch<2>(p, early_start, stream); break;
+    case 4: launch<4>(p, early_start, stream); break;
+    case 8: launch<8>(p, early_start, stream); break;
+    default: throw std::runtime_error("tridist_b200: bad stage depth");
+  }
+}
+
+}  // namespace tdb

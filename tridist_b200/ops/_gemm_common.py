@@ -201,6 +201,8 @@ def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr:
              allow_wide=env_int("TRIDIST_WIDE", 1), allow_splitk=env_int("TRIDIST_SPLITK", 1),
              # (ranks that compute together keep the tiles their exchange was measured with)
              by_rounds=1 if R == 1 else 0,
+             few_rows=1 if (R == 1 and M <= 128 and getattr(world, "kind", "") != "emulated" and
+                            not env_int("TRIDIST_MAX_CTAS", 0) and not env_int("TRIDIST_FORCE_BN", 0)) else 0,
              raster_g=env_int("TRIDIST_RASTER_G", 0),
              l2_ahead=env_int("TRIDIST_L2_AHEAD", 0),
              prof=(prof_buffer().data_ptr() if prof_buffer() is not None else 0),
@@ -274,11 +276,12 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     assert out.stride(1) == 1
+    free = bn is None and local and not max_ctas and not probe      # (the tile is nobody's choice)
     if bn is None:
         bn = choose_bn(M, N, swiglu, K=K, local=local and not max_ctas)    # (the rule counts on all SMs)
     w = plain_world()
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-           out.stride(0), bn, swiglu, a.dtype, max_ctas, probe, local)
+           out.stride(0), bn, swiglu, a.dtype, max_ctas, probe, local, free)
 
     def make():
         d = base_desc(w, 0, 1, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_PLAIN)
@@ -288,6 +291,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
         if max_ctas:
             d["max_ctas"] = max_ctas
         d["probe"] = probe
+        if not free:
+            d["few_rows"] = 0
         if not local:
             d["by_rounds"] = d["early_start"] = 0
         debug_check(d, c_bytes=tensor_extent_bytes(out))
