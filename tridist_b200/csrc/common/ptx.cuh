@@ -167,6 +167,13 @@ __device__ __forceinline__ uint4 ld_global_cg_v4(const void* p) {
                : "l"(p));
   return v;
 }
+__device__ __forceinline__ uint4 ld_global_cg_v4_hint(const void* p, uint64_t policy) {
+  uint4 v;
+  asm volatile("ld.global.cg.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p), "l"(policy));
+  return v;
+}
 // Generic address: shared memory, or global memory that bypasses L1.
 __device__ __forceinline__ uint4 ld_cg_v4(const void* p) {
   uint4 v;
@@ -262,6 +269,19 @@ __device__ __forceinline__ void bulk_load_1d(void* sdst, const void* gsrc, uint3
       :
       : "r"(smem_u32(sdst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+// The same, with a policy for the lines that it brings into L2.
+__device__ __forceinline__ void bulk_load_1d_hint(void* sdst, const void* gsrc, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+      :
+      : "r"(smem_u32(sdst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ uint64_t l2_evict_first() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
 }
 // Untiled bulk copy shared -> global (local or peer memory); both addresses 16-byte
 // aligned, size a multiple of 16 bytes. Completion is tracked by the bulk async-group.
