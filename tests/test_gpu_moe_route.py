@@ -1,0 +1,50 @@
+"""Metadata and dispatch of a small batch in one kernel, at the edges of the rule that picks it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,E,H,topk", [
+    (1, 1024, 8, 32),                        # one piece a row, most experts and rows per token
+    (147, 3, 4104, 1), (149, 300, 2056, 6),
+    (128, 1024, 64, 32), (512, 64, 4096, 8), (2048, 16, 512, 2),       # 4096 pairs: the last in one kernel
+    (513, 64, 512, 8), (2049, 16, 512, 1),   # one more: two kernels
+])
+def test_small_rounds(T, E, H, topk):
+    import test_gpu_ops
+    test_gpu_ops.test_moe_round_of_any_size(T, E, H, topk, torch.bfloat16)
+
+
+@pytest.mark.parametrize("T", [24, 600])      # one kernel, two kernels
+def test_repeated_experts_and_rows_past_the_end(T):
+    """An expert that a token names twice gets two rows; rows past the receive buffer are dropped and reported."""
+    import test_gpu_ops
+    from tridist_b200.ops import (create_moe_a2a_intra_node_context, finalize_moe_a2a_context,
+                                  moe_dispatch_intra_node_op)
+    from tridist_b200.parallel.runtime import TriDistError
+    w = test_gpu_ops._world1()
+    E, H, topk, dt = 16, 256, 8, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(1)
+    tokens = torch.randn((T, H), generator=g, device="cuda").to(dt)
+    idx = torch.randint(0, E, (T, topk), generator=g, device="cuda", dtype=torch.int32)
+    for rows in (T * topk, T * topk - 40):
+        ctx = create_moe_a2a_intra_node_context(E, H, dt, T, topk, 0, 1, BLOCK_H=H, world=w, max_recv_rows=rows)
+        total = moe_dispatch_intra_node_op(tokens, idx, ctx)
+        torch.cuda.synchronize()
+        sc = ctx.scatter_idx.flatten().long()
+        assert int(total.item()) == T * topk and int((sc < 0).sum()) == T * topk - rows
+        kept = sc >= 0
+        assert torch.equal(sc[kept].sort().values, torch.arange(rows, device="cuda"))
+        of = torch.arange(T, device="cuda").repeat_interleave(topk)
+        assert torch.equal(ctx.recv[sc[kept]], tokens[of[kept]])
+        first, e = ctx.recv_seg.flatten().long(), idx.flatten().long()
+        assert bool((sc[kept] >= first[e[kept]]).all())
+        assert torch.equal(ctx.splits.long(), torch.bincount(e, minlength=E))
+        if rows < T * topk:
+            with pytest.raises(TriDistError):
+                w.check()
+            w.clear_status()
+        else:
+            w.check()
+        finalize_moe_a2a_context(ctx)

@@ -50,6 +50,8 @@ struct alignas(16) MoeDesc {
 
 void moe_meta_launch(const MoeDesc& d, void* stream);
 void moe_dispatch_launch(const MoeDesc& d, void* stream);
+// Both: one kernel for a small batch of one rank.
+void moe_route_and_dispatch_launch(const MoeDesc& d, void* stream);
 void moe_combine_launch(const MoeDesc& d, void* stream);
 // phase 0 = meta, 1 = dispatch, 2 = combine; all ranks in ONE launch on one GPU.
 void moe_emulated_launch(const std::vector<MoeDesc>& ds, int phase, void* stream);
