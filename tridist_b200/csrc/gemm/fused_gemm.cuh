@@ -19,8 +19,8 @@
 //              communication warps reduce it and broadcast the result to all ranks
 //
 // Roles inside one CTA (320 threads, one CTA per SM):
-//   warp 0      TMA producer (one lane): smem ring of kStages {A (kMT x 128) x 64, B x 64} tiles
-//   warp 1      tcgen05.mma issuer (one lane), owns the TMEM allocation (2 accumulators)
+//   warp 0      TMA producer: smem ring of kStages {A (kMT x 128) x 64, B x 64} tiles
+//   warp 1      tcgen05.mma issuer, owns the TMEM allocation (2 accumulators)
 //   warps 2-5   epilogue: tcgen05.ld -> convert -> staged TMA stores / peer stores (+ in-epilogue reduce)
 //   warps 6-9   communication warps (AG push; AR2 reduce + broadcast + result collection)
 //
@@ -759,6 +759,12 @@ template <int BN, bool kBf16, int kCtaM, bool kStaging, int kMT>
 __global__ void __launch_bounds__(kThreads, 1)
 fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __restrict__ pv) {
   using TS = TileShape<BN, kCtaM, kStaging, kMT>;
+  // Tiles of one row block per CTA: the producer and MMA warps walk their loops as a whole and an elected lane
+  // issues. From a branch that one lane takes alone, a k-block's loads, MMAs and commit took 400 ns whatever the tile's
+  // width, more than the tensor pipe (70 to 270) or the L2 port need. us then and now, 128 x 128 tiles 1024 x 8192 x
+  // 28672 822 and 554, 128 x 256 2112 x 22016 x 4096 410 and 316, 256 x 256 339 and 276, 8192 x 12288 x 6144 946 and
+  // 810. A 512 x 256 tile's k-block keeps the tensor pipe busy for 540 ns: no gain there.
+  constexpr bool kUni = kMT == 1;
   static_assert(kCtaM == 1 || BN == 256, "CTA pairs are built for 256-wide tiles only");
   static_assert(kMT * BM * BN * 2 <= TS::kStages * TS::kStageBytes, "a slice keeps up to half its tile in the ring");
   // With pv != nullptr the launch emulates several ranks on one GPU: grid.y
@@ -784,7 +790,8 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
   // all-gather push of this CTA no longer uses the staging area; [3]: the epilogue's copy of [2]
   volatile int32_t* s_flags = s_tab + 4;
 
-  const int warp = threadIdx.x >> 5;
+  // (uniform to the compiler too, where whole warps walk the pipeline's loops)
+  const int warp = kMT == 1 ? __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0) : static_cast<int>(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // CTA pair: rank 0 of the cluster is the leader (issues the MMAs, owns the full and
   // TMEM-empty barriers the pair synchronises on).
@@ -863,10 +870,14 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
   // warp 0: TMA producer
   // ==========================================================================
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&p.tma_a);
-      tma_prefetch_desc(&p.tma_b);
-      if (p.op == OP_AG) tma_prefetch_desc(&p.tma_a_ws);
+    if (kUni || lane == 0) {
+      const bool lead = kUni ? elect_one() : true;
+      auto all = [&](bool x) { return kUni ? __all_sync(0xFFFFFFFFu, x) != 0 : x; };
+      if (lead) {
+        tma_prefetch_desc(&p.tma_a);
+        tma_prefetch_desc(&p.tma_b);
+        if (p.op == OP_AG) tma_prefetch_desc(&p.tma_a_ws);
+      }
       uint32_t stage = 0, phase = 0;
       uint64_t acc_a = 0, acc_b = 0;
       uint32_t ready_mask[kMaxRanks] = {0};   // chunks of each source already observed
@@ -892,6 +903,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
           __nanosleep(200);
           if (globaltimer_ns() - t0 > 2 * env.timeout_ns) { ok = false; break; }
         }
+        ok = all(ok);
         fence_proxy_async_smem();
       }
       WorkIter wit;
@@ -926,10 +938,11 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
                 const uint64_t tw = prof ? globaltimer_ns() : 0;
                 ok = wait_flag_ge(f, p.round, env, SITE_AG_CHUNK, (src << 16) | ck,
                                   static_cast<uint32_t>(s_budget[src]));
+                ok = all(ok);
                 if (prof) acc_a += globaltimer_ns() - tw;
                 if (ok) {
                   if (ck < 32) ready_mask[src] |= 1u << ck;
-                  if (p.arrival_ns != nullptr && ck == 0)
+                  if (lead && p.arrival_ns != nullptr && ck == 0)
                     atomicMin(reinterpret_cast<unsigned long long*>(p.arrival_ns + src),
                               static_cast<unsigned long long>(globaltimer_ns()));
                 }
@@ -956,14 +969,14 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
           tma_prefetch_l2_2d(bmap, kb * BK, b_row_pf);
           if (kCtaM == 1 && BN == 256) tma_prefetch_l2_2d(bmap, kb * BK, b_row_pf2);
         };
-        if (ahead > 0 && probe == 0)
+        if (lead && ahead > 0 && probe == 0)
           for (int kb = wi.kb0 + 1; kb < wi.kb1 && kb < wi.kb0 + ahead; ++kb) l2_request(kb);
         for (int kb = wi.kb0; kb < wi.kb1; ++kb) {
           if (probe == 1) {
             if (loads_issued >= TS::kStages) break;   // ring filled once, then idle
             ++loads_issued;
           }
-          if (ahead > 0 && kb + ahead < wi.kb1 && probe == 0) l2_request(kb + ahead);
+          if (lead && ahead > 0 && kb + ahead < wi.kb1 && probe == 0) l2_request(kb + ahead);
           if (prof && !mbar_try_wait(&empty_bar[stage], phase ^ 1u)) {
             const uint64_t tw = globaltimer_ns();
             ok = wait_mbar(&empty_bar[stage], phase ^ 1u, env, SITE_PIPE_EMPTY, stage);
@@ -971,36 +984,39 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
           } else {
             ok = wait_mbar(&empty_bar[stage], phase ^ 1u, env, SITE_PIPE_EMPTY, stage);
           }
+          ok = all(ok);
           if (!ok) break;
           pending &= ~(1u << stage);
-          uint8_t* sa = ring + stage * TS::kStageBytes;
-          uint8_t* sb = sa + TS::kABytes;
-          if constexpr (kCtaM == 2) {
-            // the leader's barrier collects the bytes of both CTAs' loads
-            if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * TS::kStageBytes);
-#pragma unroll
-            for (int h = 0; h < kMT; ++h)
-              tma_load_2d_pair(sa + h * (BM * BK * 2), amap, &full_bar[stage], kb * BK, a_row + h * BM);
-            tma_load_2d_pair(sb, bmap, &full_bar[stage], kb * BK, b_row_pair);
-          } else {
-            mbar_arrive_expect_tx(&full_bar[stage], TS::kStageBytes);
-            tma_load_2d(sa, amap, &full_bar[stage], kb * BK, a_row);
-            if (swiglu) {
-              // gate rows and the matching up rows form one BN-wide virtual tile
-              tma_load_2d(sb, bmap, &full_bar[stage], kb * BK, t.n_tile * (BN / 2));
-              tma_load_2d(sb + (BN / 2) * BK * 2, bmap, &full_bar[stage], kb * BK,
-                          up_row0 + t.n_tile * (BN / 2));
+          if (lead) {
+            uint8_t* sa = ring + stage * TS::kStageBytes;
+            uint8_t* sb = sa + TS::kABytes;
+            if constexpr (kCtaM == 2) {
+              // the leader's barrier collects the bytes of both CTAs' loads
+              if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * TS::kStageBytes);
+  #pragma unroll
+              for (int h = 0; h < kMT; ++h)
+                tma_load_2d_pair(sa + h * (BM * BK * 2), amap, &full_bar[stage], kb * BK, a_row + h * BM);
+              tma_load_2d_pair(sb, bmap, &full_bar[stage], kb * BK, b_row_pair);
             } else {
-#pragma unroll
-              for (int h = 0; h < BN / 128; ++h)
-                tma_load_2d(sb + h * 128 * BK * 2, bmap, &full_bar[stage], kb * BK, n0 + h * 128);
+              mbar_arrive_expect_tx(&full_bar[stage], TS::kStageBytes);
+              tma_load_2d(sa, amap, &full_bar[stage], kb * BK, a_row);
+              if (swiglu) {
+                // gate rows and the matching up rows form one BN-wide virtual tile
+                tma_load_2d(sb, bmap, &full_bar[stage], kb * BK, t.n_tile * (BN / 2));
+                tma_load_2d(sb + (BN / 2) * BK * 2, bmap, &full_bar[stage], kb * BK,
+                            up_row0 + t.n_tile * (BN / 2));
+              } else {
+  #pragma unroll
+                for (int h = 0; h < BN / 128; ++h)
+                  tma_load_2d(sb + h * 128 * BK * 2, bmap, &full_bar[stage], kb * BK, n0 + h * 128);
+              }
             }
           }
           pending |= 1u << stage;
           if (++stage == TS::kStages) { stage = 0; phase ^= 1u; }
         }
       }
-      if (prof) {
+      if (prof && lead) {
         prof[PROF_LOAD_FLAG_WAIT] = acc_a;
         prof[PROF_LOAD_EMPTY_WAIT] = acc_b;
       }
@@ -1023,7 +1039,9 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
   // warp 1: MMA issuer
   // ==========================================================================
   else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader && (kUni || lane == 0)) {
+      const bool lead = kUni ? elect_one() : true;
+      auto all = [&](bool x) { return kUni ? __all_sync(0xFFFFFFFFu, x) != 0 : x; };
       constexpr uint32_t idesc = umma_idesc_f16(kBf16, BM * kCtaM, BN);
       uint32_t stage = 0, phase = 0;
       uint64_t acc_f = 0, acc_t = 0;
@@ -1040,6 +1058,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
       constexpr uint64_t kDescRows = static_cast<uint64_t>((BM * BK * 2) >> 4);   // next 128 rows of A
       // four MMAs of one 64-wide k-block into accumulator d_tmem; `fresh` overwrites it
       auto mma4 = [&](uint32_t d_tmem, uint64_t da, uint64_t db, bool fresh) {
+        if (!lead) return;
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k) {
           // +32 bytes per K step inside the 128-byte swizzle row
@@ -1053,27 +1072,29 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
       };
       // frees the smem stage (in both CTAs of a pair) when the MMAs issued so far retire
       auto commit_stage = [&](uint32_t s) {
+        if (!lead) return;
         if constexpr (kCtaM == 2) umma_commit_pair_both(&empty_bar[s]);
         else umma_commit(&empty_bar[s]);
       };
       // accumulator complete (each CTA of a pair reads its own 128 rows)
       auto commit_acc = [&](int b) {
+        if (!lead) return;
         if constexpr (kCtaM == 2) umma_commit_pair_both(&tmem_full_bar[b]);
         else umma_commit(&tmem_full_bar[b]);
       };
       auto wait_full = [&](uint32_t s, uint32_t ph) -> bool {
-        if (mbar_try_wait(&full_bar[s], ph)) return true;
+        if (all(mbar_try_wait(&full_bar[s], ph))) return true;
         const uint64_t tw = prof ? globaltimer_ns() : 0;
         const bool r = wait_mbar(&full_bar[s], ph, env, SITE_PIPE_FULL, s);
         if (prof) acc_f += globaltimer_ns() - tw;
-        return r;
+        return all(r);
       };
       auto wait_acc_free = [&](int b, uint32_t par) -> bool {
-        if (mbar_try_wait(&tmem_empty_bar[b], par)) return true;
+        if (all(mbar_try_wait(&tmem_empty_bar[b], par))) return true;
         const uint64_t tw = prof ? globaltimer_ns() : 0;
         const bool r = wait_mbar(&tmem_empty_bar[b], par, env, SITE_TMEM_EMPTY, b);
         if (prof) acc_t += globaltimer_ns() - tw;
-        return r;
+        return all(r);
       };
       WorkIter wit;
       WorkItem wi;
@@ -1099,8 +1120,10 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
               ++kblocks_done;
               if (probe == 2) {
                 // operand-feed ceiling: hand the stage straight back to the producer(s)
-                mbar_arrive(&empty_bar[stage]);
-                if constexpr (kCtaM == 2) mbar_arrive_cluster(&empty_bar[stage], 1u);
+                if (lead) {
+                  mbar_arrive(&empty_bar[stage]);
+                  if constexpr (kCtaM == 2) mbar_arrive_cluster(&empty_bar[stage], 1u);
+                }
                 if (++stage == TS::kStages) { stage = 0; phase ^= 1u; }
                 continue;
               }
@@ -1149,8 +1172,10 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
             if (probe != 0) {
               ++kblocks_done;
               if (probe == 2) {
-                mbar_arrive(&empty_bar[stage]);
-                mbar_arrive_cluster(&empty_bar[stage], 1u);
+                if (lead) {
+                  mbar_arrive(&empty_bar[stage]);
+                  mbar_arrive_cluster(&empty_bar[stage], 1u);
+                }
                 if (j == nkb - 1) { commit_acc(0); commit_acc(1); }
                 if (++stage == TS::kStages) { stage = 0; phase ^= 1u; }
                 continue;
@@ -1168,11 +1193,11 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         }
         ++it;
       }
-      if (prof) {
+      if (prof && lead) {
         prof[PROF_MMA_FULL_WAIT] = acc_f;
         prof[PROF_MMA_TMEM_WAIT] = acc_t;
       }
-      if (!ok) {
+      if (!ok && lead) {
         // Unwinding: MMAs already issued must retire before TMEM is freed.
         if constexpr (kCtaM == 2) umma_commit_pair_local(drain_bar);
         else umma_commit(drain_bar);
