@@ -165,6 +165,46 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
   return 2;
 }
 
+// Local launches: which of the four tiles, by the time expected of it. A round of tiles takes so many us a
+// k-block, a cut last round its share of them and the parking and adding of the partials, 512 x 256 tiles their
+// epilogue in every round (both accumulators are in use), any of them no less than the operands take from DRAM.
+// The constants are fitted to 64 shapes of 192 to 8192 rows, each of the tiles timed in turn (the tile chosen was 0.6 %
+// slower than the fastest on average, 7 % with the rule by rounds alone), but for 4 % more on 256 x 256 tiles: in
+// long runs under the power cap their operand traffic costs that much. us with 128 x 128, 128 x 256, 256 x 256 and 512 x 256
+// tiles (rows x N x K): 384 x 3328 x 1584 16.8, 23.6, 21.6, 25.2; 320 x 28672 x 8192 236, 160, 171, 171; 2112 x 22016 x
+// 4096 485, 316, 276, 314; 1728 x 12288 x 12288 656, 416, 370, 446; 8192 x 6144 x 12288 774 as 512 x 256, 800 as 256 x 256.
+static GemmPlanDesc fit_tile(GemmPlanDesc d) {
+  if (!d.fit_tile || d.R != 1 || d.sched != SCHED_NATURAL || d.max_ctas > 0 || d.probe != 0) return d;
+  struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi; };
+  const bool swiglu = d.epi == EPI_SWIGLU;
+  const Tile tiles[4] = {{128, 1, 0, 0.375, 8.0, 5.0, 0.0},
+                         {256, 1, 0, 0.47, 10.0, 6.5, 0.0},
+                         {256, 2, 1, 0.42, 12.0, 6.0, 0.0},
+                         {256, 4, 1, 0.78, 12.0, 12.0, swiglu ? 6.0 : 3.5}};
+  const int mt = (d.M + BM - 1) / BM, kb = (d.K + BK - 1) / BK;
+  const double dram = (static_cast<double>(d.N) * (swiglu ? 2 : 1) * d.K + static_cast<double>(d.M) * (d.K + d.N)) * 2 / 6.3e6;
+  double best_us = -1;
+  GemmPlanDesc best = d;
+  for (const Tile& t : tiles) {
+    if (swiglu && t.bn != 256) continue;
+    if ((t.pairs && (!d.allow_pair || mt < 2)) || (t.blocks == 4 && (!d.allow_wide || mt < 4))) continue;
+    const int bn_out = swiglu ? t.bn / 2 : t.bn, g = t.pairs ? 74 : 148;
+    const int64_t n = static_cast<int64_t>((mt + t.blocks - 1) / t.blocks) * ((d.N + bn_out - 1) / bn_out);
+    const int left = static_cast<int>(n % g), s = d.allow_splitk ? slices_for(left, g, kb) : 1;
+    const double whole = kb * t.per_kb;
+    double us = static_cast<double>(n / g) * (whole + t.epi);
+    if (left > 0) us += (s == 1 ? whole : std::min(whole, whole / s + t.meet)) + t.epi;
+    us = std::max(us, dram) + t.fixed;
+    if (best_us >= 0 && us >= best_us) continue;
+    best_us = us;
+    best.bn = t.bn;
+    best.allow_pair = t.pairs;
+    best.allow_wide = t.blocks == 4 ? 1 : 0;
+    best.by_rounds = 0;
+  }
+  return best;
+}
+
 // Everything the tile schedule depends on (shared by plan creation and the host-side dump).
 static void fill_schedule_fields(const GemmPlanDesc& d, int cta_m, int cta_mt, GemmParams& p) {
   const int bn_out = (d.epi == EPI_SWIGLU) ? d.bn / 2 : d.bn;
@@ -265,7 +305,8 @@ static SplitScratch bind_sk_scratch(GemmParams& p, int slots, cudaStream_t strea
   return sc;
 }
 
-std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& d, int sms) {
+std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& desc, int sms) {
+  const GemmPlanDesc d = fit_tile(desc);
   if (d.sched == SCHED_LIST) throw std::runtime_error("tridist_b200: a tile list is its own schedule");
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
@@ -292,7 +333,8 @@ std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& d
 
 // The K ranges of the tiles that are cut along K: {scheduling position, first CTA of the worker,
 // slice, slices, first k-block, end k-block} for every worker that takes part.
-std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& d, int sms) {
+std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& desc, int sms) {
+  const GemmPlanDesc d = fit_tile(desc);
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   const int cta_m = choose_cta_m(d);
@@ -309,7 +351,8 @@ std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& d, int sms) {
   return out;
 }
 
-std::vector<std::string> plan_check(const GemmPlanDesc& d, const PlanExtents& e, int sms) {
+std::vector<std::string> plan_check(const GemmPlanDesc& desc, const PlanExtents& e, int sms) {
+  const GemmPlanDesc d = fit_tile(desc);
   std::vector<std::string> bad;
   auto need = [&](const char* what, int64_t want, int64_t have, const char* unit) {
     if (have > 0 && want > have)
@@ -393,7 +436,8 @@ std::vector<std::string> plan_check(const GemmPlanDesc& d, const PlanExtents& e,
   return bad;
 }
 
-int64_t gemm_plan_create(const GemmPlanDesc& d) {
+int64_t gemm_plan_create(const GemmPlanDesc& desc) {
+  const GemmPlanDesc d = fit_tile(desc);
   if (d.R < 1 || d.R > kMaxRanks) throw std::runtime_error("tridist_b200: 1 <= R <= 8 required");
   if (d.bn != 128 && d.bn != 256) throw std::runtime_error("tridist_b200: BN must be 128 or 256");
   if (d.epi == EPI_SWIGLU && d.bn != 256)
@@ -577,6 +621,10 @@ static int resident_ctas() {
 
 static bool plan_uses_staging(const GemmParams& p) {
   // operators that ship data to other ranks (epilogue tiles, all-gather push) need the staging area
+  // Local 256 x 256 tiles of a short K, whose epilogue shows, leave through it too; a long K rather has the seventh ring
+  // stage. us with and without (rows x N x K): 1984 x 8192 x 3696 108 and 118, 2048 x 9856 x 2656 89 and 101, 2432 x 4096
+  // x 1376 37 and 42; 2112 x 22016 x 4096 316 and 300, 8192 x 12288 x 6144 828 and 810.
+  if (p.R == 1 && p.cta_m == 2 && p.cta_mt == 1 && p.k_blocks < 60) return true;
   return p.R > 1 && (p.op == OP_RS || p.op == OP_AR1 || p.op == OP_AR2 || p.op == OP_AG);
 }
 

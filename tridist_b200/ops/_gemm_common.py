@@ -186,6 +186,9 @@ def read_prof(n_ctas: int = 148) -> Dict[str, Dict[str, float]]:
 def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr: int, ldc: int,
               M: int, N: int, K: int, bn: int, op: int) -> Dict:
     assert a.stride(1) == 1 and b.stride(1) == 1, "operands must be row-major with unit inner stride"
+    # one rank: the tile (or, for few rows, the kernel) is the plan's own choice unless the environment makes it
+    free = (R == 1 and getattr(world, "kind", "") != "emulated" and not env_int("TRIDIST_MAX_CTAS", 0) and
+            not env_int("TRIDIST_FORCE_BN", 0))
     d = dict(op=op, epi=EPI_STORE, sched=SCHED_NATURAL, bn=bn, bf16=is_bf16(a.dtype), rank=rank, R=R,
              M=M, N=N, K=K, a=a.data_ptr(), a_rows=a.shape[0], lda=a.stride(0),
              b=b.data_ptr(), b_rows=b.shape[0], ldb=b.stride(0), c=c_ptr, ldc=ldc,
@@ -201,8 +204,7 @@ def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr:
              allow_wide=env_int("TRIDIST_WIDE", 1), allow_splitk=env_int("TRIDIST_SPLITK", 1),
              # (ranks that compute together keep the tiles their exchange was measured with)
              by_rounds=1 if R == 1 else 0,
-             few_rows=1 if (R == 1 and M <= 128 and getattr(world, "kind", "") != "emulated" and
-                            not env_int("TRIDIST_MAX_CTAS", 0) and not env_int("TRIDIST_FORCE_BN", 0)) else 0,
+             few_rows=1 if (free and M <= 128) else 0, fit_tile=1 if free else 0,
              raster_g=env_int("TRIDIST_RASTER_G", 0),
              l2_ahead=env_int("TRIDIST_L2_AHEAD", 0),
              prof=(prof_buffer().data_ptr() if prof_buffer() is not None else 0),
@@ -292,7 +294,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
             d["max_ctas"] = max_ctas
         d["probe"] = probe
         if not free:
-            d["few_rows"] = 0
+            d["few_rows"] = d["fit_tile"] = 0
         if not local:
             d["by_rounds"] = d["early_start"] = 0
         debug_check(d, c_bytes=tensor_extent_bytes(out))
