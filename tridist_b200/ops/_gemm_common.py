@@ -108,20 +108,37 @@ class PlanCache:
     def __init__(self, capacity: int = 64):
         self.capacity = capacity
         self._d: "OrderedDict[tuple, int]" = OrderedDict()
-        self.hits = self.misses = self.evictions = 0
+        self._hits = self.misses = self.evictions = 0
         self._warned = False
+        self.recent = None       # native: calls of one rank whose plan is known (see remember)
+
+    @property
+    def hits(self) -> int:
+        return self._hits + (self.recent.hits if self.recent is not None else 0)
+
+    def remember(self, a, b, c, tag: int, key: tuple) -> None:
+        """From now on ``recent.launch(a, b, c, tag, round)`` launches the plan of ``key`` by itself, until the
+        plan leaves the cache. ``tag``: what of the call is not in the tensors."""
+        if self.recent is None:
+            self.recent = native().RecentCalls()
+        self.recent.remember(a, b, c, tag, self._d[key], key)
 
     def get(self, key: tuple, make) -> int:
         pid = self._d.get(key)
         if pid is not None:
             self._d.move_to_end(key)
-            self.hits += 1
+            self._hits += 1
             return pid
         self.misses += 1
         pid = make()
+        if self.recent is not None:
+            for used in self.recent.drain():
+                self._d.move_to_end(used)
         self._d[key] = pid
         if len(self._d) > self.capacity:
             _, old = self._d.popitem(last=False)
+            if self.recent is not None:
+                self.recent.forget(old)
             native().gemm_plan_destroy(old)
             self.evictions += 1
             if self.evictions >= 4 * self.capacity and not self._warned:
@@ -137,6 +154,8 @@ class PlanCache:
         for pid in self._d.values():
             C.gemm_plan_destroy(pid)
         self._d.clear()
+        if self.recent is not None:
+            self.recent.clear()
 
 
 PROF_SLOTS = ["load_flag_wait", "load_empty_wait", "mma_full_wait", "mma_tmem_wait", "epi_busy", "epi_publish",

@@ -306,7 +306,10 @@ def _plan(ctx, a, b, c, swiglu=False):
             debug_check(d, c_bytes=tensor_extent_bytes(c))
         return native().gemm_plan_create(d)
 
-    return ctx.plans.get(key, make)
+    pid = ctx.plans.get(key, make)
+    if R == 1 and baked_table is None and not ctx.observe and not isinstance(ctx.world, EmulatedWorld):
+        ctx.plans.remember(a, b, c, 1 if swiglu else 0, key)
+    return pid
 
 
 def _check_args(a, b, c, ctx):
@@ -337,6 +340,12 @@ def ag_gemm_intra_node_op(a, b, c, ctx, skip_comm=False, order_table: Optional[t
     """
     if isinstance(ctx.world, CpuWorld):
         return cpu_backend.ag_gemm(a, b, c, ctx, skip_comm, fuse_swiglu)
+    recent = ctx.plans.recent       # one rank's calls whose plan is known (checked when it was made)
+    if recent is not None and not (skip_comm or comm_only or ctx.observe or order_table is not None):
+        rnd = next_round(ctx.flag_round, "all-gather context")
+        if recent.launch(a, b, c, 1 if fuse_swiglu else 0, rnd):
+            ctx.flag_round = rnd
+            return c
     _check_args(a, b, c, ctx)
     if not skip_comm:
         ctx.flag_round = next_round(ctx.flag_round, "all-gather context")

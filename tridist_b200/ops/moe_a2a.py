@@ -139,7 +139,7 @@ def create_moe_a2a_intra_node_context(num_experts, hidden, dtype, max_tokens, to
 def _handle(ctx):
     h = ctx._handle
     if h is None:
-        h = native().MoeHandle(_desc(ctx, parity=0), _desc(ctx, parity=1))
+        h = native().MoeHandle(_desc(ctx, parity=0), _desc(ctx, parity=1), ctx.max_tokens)
         object.__setattr__(ctx, "_handle", h)
     return h
 
@@ -185,10 +185,11 @@ def moe_dispatch_intra_node_op(tokens, topk_idx, ctx, component="full"):
         raise ValueError(f"unknown component {component!r}")
     if isinstance(ctx.world, CpuWorld):
         return cpu_backend.moe_dispatch(tokens, topk_idx, ctx, component)
-    T = _check_dispatch(tokens, topk_idx, ctx)
-    ctx.meta_round = next_round(ctx.meta_round, "MoE context")
-    _handle(ctx).dispatch(ctx.meta_round, ctx.world.timeout_ns, tokens.data_ptr(), topk_idx.data_ptr(), T,
-                          component == "full")
+    rnd = next_round(ctx.meta_round, "MoE context")
+    if not (ctx._handle or _handle(ctx)).dispatch(rnd, ctx.world.timeout_ns, tokens, topk_idx, component == "full"):
+        _check_dispatch(tokens, topk_idx, ctx)
+        raise ValueError("tridist_b200: tokens and topk_idx do not fit the MoE context")
+    object.__setattr__(ctx, "meta_round", rnd)
     return ctx.recv_total_t
 
 
@@ -196,12 +197,12 @@ def moe_combine_intra_node_op(ctx, topk_idx, output, topk_weights=None):
     """Pull-combine of the expert outputs; must follow a dispatch of the same round."""
     if isinstance(ctx.world, CpuWorld):
         return cpu_backend.moe_combine(ctx, topk_idx, output, topk_weights)
-    T = topk_idx.shape[0]
-    assert output.shape[0] == T and output.shape[1] == ctx.hidden and output.is_contiguous()
-    if topk_weights is not None:
-        assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
-    _handle(ctx).combine(ctx.meta_round, ctx.world.timeout_ns, topk_idx.data_ptr(),
-                         topk_weights.data_ptr() if topk_weights is not None else 0, output.data_ptr(), T)
+    if not (ctx._handle or _handle(ctx)).combine(ctx.meta_round, ctx.world.timeout_ns, topk_idx, topk_weights, output):
+        T = topk_idx.shape[0]
+        assert output.shape[0] == T and output.shape[1] == ctx.hidden and output.is_contiguous()
+        if topk_weights is not None:
+            assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
+        raise ValueError("tridist_b200: output and topk_weights do not fit the MoE context")
     return output
 
 
