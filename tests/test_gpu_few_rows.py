@@ -1,4 +1,4 @@
-"""The GEMM for at most 128 rows (csrc/gemm/skinny_gemm.cuh) on one GPU, at the edges of its layout."""
+"""The GEMM for few rows (csrc/gemm/skinny_gemm.cuh) on one GPU, at the edges of its layout."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -121,3 +121,37 @@ def test_few_rows_of_a_context_follow_the_kernel_in_front():
     err = (x[0].double() - refs[6].double()).norm() / refs[6].double().norm()
     assert err < 6 * 2.0 ** -8
     finalize_gemm_ar_context(ctx)
+
+
+@pytest.mark.parametrize("M,N,K,swiglu,cluster", [
+    (129, 8, 64, False, 1), (160, 264, 136, False, 1), (256, 6144, 592, False, 1), (192, 40000, 512, False, 1),
+    (150, 4096, 4104, False, 2), (256, 11008, 4096, False, 2), (224, 1416, 4104, True, 2), (256, 8192, 28672, False, 4),
+    (200, 48, 8200, False, 4), (193, 1664, 12288, False, 4), (130, 20000, 320, True, 1),
+])
+def test_two_blocks_of_rows(M, N, K, swiglu, cluster, monkeypatch):
+    """129 to 256 rows, also where the plan would rather take the general kernel."""
+    from tridist_b200.ops._gemm_common import gemm_nt
+    from tridist_b200.parallel.runtime import native
+    C = native()
+    lay = C.skinny_layout(M, N, K, swiglu, 148)
+    assert (lay["cluster"], lay["mb"]) == (cluster, 2)
+    create = C.gemm_plan_create
+    monkeypatch.setattr(C, "gemm_plan_create", lambda d: create(dict(d, few_rows=2)))
+    for dt in (torch.float16, torch.bfloat16):
+        a, b = _rand((M, K), 8, dt), _rand((2 * N if swiglu else N, K), 9, dt)
+        plane = torch.full((M + 1, N + 8), 7.0, dtype=dt, device="cuda")
+        out = plane[:M, :N]
+        for _ in range(3):
+            out.zero_()
+            gemm_nt(a, b, out=out, swiglu=swiglu)
+        torch.cuda.synchronize()
+        assert bool((plane[M] == 7.0).all()) and bool((plane[:, N:] == 7.0).all())
+        exact = a.double() @ b.double().t()
+        bound = _bound(a, b, exact, dt)
+        if swiglu:
+            gate, up = exact[:, :N], exact[:, N:]
+            exact = F.silu(gate) * up
+            e = K * 2.0 ** -23 * (a.abs().double() @ b.abs().double().t())
+            bound = (exact.abs() * (2.0 ** -11 if dt == torch.float16 else 2.0 ** -8) * 1.01 + exact.abs() * 2.0 ** -18 +
+                     1.1 * e[:, :N] * up.abs() + F.silu(gate).abs() * e[:, N:] + 2.0 ** -24)
+        assert bool(((out.double() - exact).abs() <= bound).all())

@@ -10,7 +10,8 @@ def test_layout_holds_for_every_shape(seed):
     from tridist_b200.parallel.runtime import native
     rnd = random.Random(seed)
     shapes = [(1, 8, 8, 0), (128, 8, 64, 1), (64, 4096, 1376, 0), (65, 8192, 3584, 0), (128, 3584, 8192, 1), (128, 106496, 16384, 0)]
-    shapes += [(rnd.randint(1, 128), 8 * rnd.randint(1, rnd.choice([4, 300, 2400, 14000])), 8 * rnd.randint(1, rnd.choice([20, 4000])),
+    shapes += [(129, 8, 64, 0), (256, 12288, 24576, 0), (200, 53248, 16384, 1), (192, 16384, 8192, 1)]
+    shapes += [(rnd.randint(1, 256), 8 * rnd.randint(1, rnd.choice([4, 300, 2400, 14000])), 8 * rnd.randint(1, rnd.choice([20, 4000])),
                 rnd.randint(0, 1)) for _ in range(150)]
     for M, N, K, swiglu in shapes:
         p = native().skinny_layout(M, N, K, bool(swiglu), 148)
@@ -27,17 +28,17 @@ def test_layout_holds_for_every_shape(seed):
         assert min(ranges) >= 1, what
         # shared memory: whole swizzle groups, A's 128 rows of the last k-block inside the pad, TMA's limits
         assert p["wr"] % 8 == 0 and p["wr"] <= p["nb"] and p["nb"] % 16 == 0 and p["wr"] <= 256, what
-        assert p["ar"] % 8 == 0 and M <= p["ar"] <= 128 and 32 * p["warps"] >= M, what
+        assert p["ar"] % 8 == 0 and M <= p["ar"] <= 256 and 32 * p["warps"] >= M and p["mb"] == -(-M // 128), what
         block = (p["ar"] + p["nb"] * p["boxes"]) * 128
         assert p["kw"] in (1, 2, 4, 8) and p["stage_bytes"] == p["kw"] * block and block % 1024 == 0, what
         ring = p["stages"] * p["stage_bytes"]
         assert 1 <= p["stages"] <= 16, what
-        assert (p["kw"] - 1) * p["ar"] * 128 + 128 * 128 <= p["stage_bytes"] + p["pad"], what
+        assert (p["kw"] - 1) * p["ar"] * 128 + p["mb"] * 128 * 128 <= p["stage_bytes"] + p["pad"], what
         xbuf = (cl - 1) * p["boxes"] * p["own"] * 2 * 32 * p["warps"] * 16
-        assert ring + p["pad"] + xbuf <= p["smem_bytes"] <= 225 * 1024, what
+        assert (max(ring + p["pad"], xbuf) if p["in_ring"] else ring + p["pad"] + xbuf) <= p["smem_bytes"] <= 225 * 1024, what
         # tensor memory and the MMA's shape
         bufs = 2 if p["shares"] > p["workers"] else 1
         assert p["mma_n"] % 16 == 0 and 16 <= p["mma_n"] <= 256 and p["acc_cols"] >= p["mma_n"], what
-        assert bufs * p["accs"] * p["acc_cols"] <= p["tmem_cols"] <= 512 and p["tmem_cols"] & (p["tmem_cols"] - 1) == 0, what
+        assert p["mb"] * bufs * p["accs"] * p["acc_cols"] <= p["tmem_cols"] <= 512 and p["tmem_cols"] & (p["tmem_cols"] - 1) == 0, what
         assert 1 <= p["accs"] <= max(1, min(ranges) // 16), what
         assert p["accs"] <= -(-min(ranges) // p["kw"]), what

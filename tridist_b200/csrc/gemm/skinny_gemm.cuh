@@ -1,4 +1,4 @@
-// C = A @ B^T for few rows of A (at most 128, a decode batch): the time is that of reading B once.
+// C = A @ B^T for few rows of A (at most 256, a decode batch): the time is that of reading B once.
 //
 // A worker is a cluster of 1, 2, 4 or 8 CTAs. It takes a share of B's rows, an even run of 8-row groups, whole, and
 // its CTAs a range of K each. Rows of A are re-read through L2 by every worker; what a CTA reads in all bounds
@@ -11,7 +11,7 @@
 // 1376 14.7 and 7.6, 128 x 8192 x 3584 23 and 15.5, 128 x 2 x 3584 x 8192 with SwiGLU 35.6 and 29.
 //
 // Roles (224 threads): warp 0 loads B, warp 6 A, warp 1 multiplies and owns the tensor memory, warps 2-5 store,
-// one TMEM lane quarter (32 rows) each. A long range of K is summed in up to four accumulators, one run of it each, that
+// one TMEM lane quarter (32 rows) each of every 128-row block of A. A long range of K is summed in up to four accumulators, one run of it each, that
 // the epilogue adds in order. Loads and MMAs are issued by an elected lane of a warp whose control flow is
 // uniform, with a stage of kW k-blocks unrolled: a k-block is 32 to 128 cycles of the tensor pipe for so few
 // rows, and a loop that issues it from one diverged lane takes 400 or more.
@@ -33,9 +33,10 @@ template <int kW>
 __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __grid_constant__ SkinnyParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* const ring = smem;
-  uint8_t* const xbuf = smem + p.stages * p.stage_bytes + p.pad;      // parts from the other CTAs of the cluster
+  // parts from the other CTAs of the cluster
+  uint8_t* const xbuf = p.parts_in_ring ? ring : smem + p.stages * p.stage_bytes + p.pad;
   __shared__ __align__(8) uint64_t full_bar[kSkinnyMaxStages], empty_bar[kSkinnyMaxStages], acc_full[2], acc_empty[2],
-      x_full, drain_bar;
+      x_full, x_ready, drain_bar;
   __shared__ uint32_t tmem_slot;
 
   const int warp = __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -54,7 +55,8 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 4);
     }
-    mbar_init(&x_full, max(1, (cluster - 1) * p.warps));
+    mbar_init(&x_full, max(1, (cluster - 1) * min(4, p.warps)));
+    mbar_init(&x_ready, max(1, cluster - 1));
     mbar_init(&drain_bar, 1);
     mbar_fence_init();
   }
@@ -145,6 +147,8 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
     const uint64_t stage_step = static_cast<uint64_t>(p.stage_bytes >> 4);
     const uint32_t idesc = umma_idesc_f16(p.bf16 != 0, 128, p.mma_n);
     const int al2 = p.accs_log2, acc_cols = p.acc_cols;
+    const bool two_blocks = p.mb == 2;
+    const uint32_t d_block = static_cast<uint32_t>(acc_cols << al2);      // from block 0's accumulators to block 1's
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -155,7 +159,7 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
       ok = __all_sync(0xFFFFFFFFu, ok) != 0;
       if (!ok) break;
       tc_fence_after_sync();
-      uint32_t d = tmem + static_cast<uint32_t>((buf << al2) * acc_cols);
+      uint32_t d = tmem + static_cast<uint32_t>(buf * p.mb) * d_block;
       int acc = 0, acc_end = steps >> al2;
       uint32_t keep = 0u;                           // 0: the next MMA overwrites its accumulator
       for (int i = 0; i < steps; ++i) {
@@ -179,6 +183,11 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
 #pragma unroll
             for (int k = 0; k < 4; ++k)
               umma_f16_ss(d, da + j * a_step + k * 2, db + j * b_step + k * 2, idesc, (j | k) ? 1u : keep);
+            if (two_blocks) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                umma_f16_ss(d + d_block, da + j * a_step + 1024 + k * 2, db + j * b_step + k * 2, idesc, (j | k) ? 1u : keep);
+            }
           }
           umma_commit(&empty_bar[stage]);
         }
@@ -205,8 +214,6 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
     griddep_wait();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
     const int q = warp & 3;                         // TMEM lane quarter
-    const int token = q * 32 + lane;
-    const bool row_ok = token < p.M;
     const bool warp_on = q < p.warps;
     const int accs = 1 << p.accs_log2, acc_cols = p.acc_cols, swiglu = p.swiglu;
     const EvenRuns share = p.share;
@@ -215,7 +222,6 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
     // xbuf: [source, the owner left out][gate, up][group of the owner's run][two 16-byte halves][row]
     const int rows = p.warps * 32;
     const int x_half = rows * 16, x_group = 2 * x_half, x_part = p.own * x_group, x_src = (swiglu ? 2 : 1) * x_part;
-    uint8_t* const c_row = reinterpret_cast<uint8_t*>(p.c) + static_cast<int64_t>(token) * p.ldc * 2;
     // sum of the accumulators, columns [col, col + 8 G)
     auto take = [&](uint32_t t, int col, auto& x) {
       constexpr int kCols = sizeof(x) / 4;
@@ -239,32 +245,44 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
       ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t t = tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * accs * acc_cols);
+      const uint32_t t0 = tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * p.mb * accs * acc_cols);
       const int g_lo = share.start(v);
       const int n = share.start(v + 1) - g_lo;      // groups of the share
       auto owned = [&](int r) { return (n * r) >> cl2; };      // first of them that CTA r of the cluster adds up
       if (warp_on) {
         if (cluster > 1) {
           // (a cluster has one share: the parts' buffer is written once)
+          if (p.parts_in_ring) {
+            // this CTA's loads and MMAs are through with its ring; the others' must be before it writes there
+            if (q == 0 && lane == 0)
+              for (int o = 1; o < cluster; ++o) mbar_arrive_cluster(&x_ready, static_cast<uint32_t>((sub + o) & (cluster - 1)));
+            __syncwarp();
+            if (lane == 0) ok = wait_mbar(&x_ready, 0u, env, SITE_SPLITK, sub);
+            ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
+            if (!ok) break;
+          }
           for (int o = 1; o < cluster; ++o) {
             const int dst = (sub + o) & (cluster - 1);
             const int lo = owned(dst), hi = owned(dst + 1);
-            const uint32_t base = cluster_smem_addr(xbuf + (sub < dst ? sub : sub - 1) * x_src + token * 16, static_cast<uint32_t>(dst));
-            for (int h = 0; h < (swiglu ? 2 : 1); ++h) {
-              auto send = [&](int g, auto& x) {
-                take(t, h * up_col + g * 8, x);
+            for (int m = 0; m < p.mb && m * 4 + q < p.warps; ++m) {
+              const uint32_t t = t0 + static_cast<uint32_t>(m * accs * acc_cols);
+              const uint32_t base = cluster_smem_addr(xbuf + (sub < dst ? sub : sub - 1) * x_src + (m * 128 + q * 32 + lane) * 16, static_cast<uint32_t>(dst));
+              for (int h = 0; h < (swiglu ? 2 : 1); ++h) {
+                auto send = [&](int g, auto& x) {
+                  take(t, h * up_col + g * 8, x);
 #pragma unroll
-                for (int k = 0; k < static_cast<int>(sizeof(x) / 32); ++k) {
-                  const uint32_t to = base + static_cast<uint32_t>(h * x_part + (g + k - lo) * x_group);
-                  st_cluster_v4(to, x[8 * k], x[8 * k + 1], x[8 * k + 2], x[8 * k + 3]);
-                  st_cluster_v4(to + static_cast<uint32_t>(x_half), x[8 * k + 4], x[8 * k + 5], x[8 * k + 6], x[8 * k + 7]);
+                  for (int k = 0; k < static_cast<int>(sizeof(x) / 32); ++k) {
+                    const uint32_t to = base + static_cast<uint32_t>(h * x_part + (g + k - lo) * x_group);
+                    st_cluster_v4(to, x[8 * k], x[8 * k + 1], x[8 * k + 2], x[8 * k + 3]);
+                    st_cluster_v4(to + static_cast<uint32_t>(x_half), x[8 * k + 4], x[8 * k + 5], x[8 * k + 6], x[8 * k + 7]);
+                  }
+                };
+                int g = lo;
+                for (float x[16]; g + 2 <= hi; g += 2) send(g, x);
+                if (g < hi) {
+                  float x[8];
+                  send(g, x);
                 }
-              };
-              int g = lo;
-              for (float x[16]; g + 2 <= hi; g += 2) send(g, x);
-              if (g < hi) {
-                float x[8];
-                send(g, x);
               }
             }
             __syncwarp();                           // the warp's stores before the arrival that publishes them
@@ -276,65 +294,71 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
           fence_acq_rel_cluster();
         }
         const int lo = owned(sub), hi = owned(sub + 1);
-        // the sum over the K ranges, in their order, of the gate (h = 0) or up columns of the groups from g on
-        auto sum = [&](int h, int g, auto& x) {
-          constexpr int kGroups = sizeof(x) / 32;
-          if (cluster == 1) {
-            take(t, h * up_col + g * 8, x);
-            return;
-          }
-          float mine[8 * kGroups];
-          take(t, h * up_col + g * 8, mine);
+        for (int m = 0; m < p.mb && m * 4 + q < p.warps; ++m) {
+          const uint32_t t = t0 + static_cast<uint32_t>(m * accs * acc_cols);
+          const int token = m * 128 + q * 32 + lane;
+          const bool row_ok = token < p.M;
+          uint8_t* const c_row = reinterpret_cast<uint8_t*>(p.c) + static_cast<int64_t>(token) * p.ldc * 2;
+          // the sum over the K ranges, in their order, of the gate (h = 0) or up columns of the groups from g on
+          auto sum = [&](int h, int g, auto& x) {
+            constexpr int kGroups = sizeof(x) / 32;
+            if (cluster == 1) {
+              take(t, h * up_col + g * 8, x);
+              return;
+            }
+            float mine[8 * kGroups];
+            take(t, h * up_col + g * 8, mine);
 #pragma unroll
-          for (int j = 0; j < 8 * kGroups; ++j) x[j] = 0.f;
-          const uint8_t* from = xbuf + h * x_part + (g - lo) * x_group + token * 16;
+            for (int j = 0; j < 8 * kGroups; ++j) x[j] = 0.f;
+            const uint8_t* from = xbuf + h * x_part + (g - lo) * x_group + token * 16;
 #pragma unroll 1
-          for (int s = 0; s < cluster; ++s) {
+            for (int s = 0; s < cluster; ++s) {
 #pragma unroll
-            for (int k = 0; k < 2 * kGroups; ++k) {
-              const float4 y = s == sub ? make_float4(mine[4 * k], mine[4 * k + 1], mine[4 * k + 2], mine[4 * k + 3])
-                                        : *reinterpret_cast<const float4*>(from + k * x_half);
-              x[4 * k] += y.x;
-              x[4 * k + 1] += y.y;
-              x[4 * k + 2] += y.z;
-              x[4 * k + 3] += y.w;
+              for (int k = 0; k < 2 * kGroups; ++k) {
+                const float4 y = s == sub ? make_float4(mine[4 * k], mine[4 * k + 1], mine[4 * k + 2], mine[4 * k + 3])
+                                          : *reinterpret_cast<const float4*>(from + k * x_half);
+                x[4 * k] += y.x;
+                x[4 * k + 1] += y.y;
+                x[4 * k + 2] += y.z;
+                x[4 * k + 3] += y.w;
+              }
+              if (s != sub) from += x_src;
             }
-            if (s != sub) from += x_src;
-          }
-        };
-        auto finish = [&](int g, auto& x, auto& u) {
-          constexpr int kCols = sizeof(x) / 4;
-          sum(0, g, x);
-          if (swiglu) {
-            sum(1, g, u);
+          };
+          auto finish = [&](int g, auto& x, auto& u) {
+            constexpr int kCols = sizeof(x) / 4;
+            sum(0, g, x);
+            if (swiglu) {
+              sum(1, g, u);
 #pragma unroll
-            for (int j = 0; j < kCols; ++j) x[j] = skinny_silu(x[j]) * u[j];
-          }
-          uint32_t w[kCols / 2];
-          if (bf16) {
-#pragma unroll
-            for (int j = 0; j < kCols / 2; ++j) {
-              __nv_bfloat162 y = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-              w[j] = *reinterpret_cast<uint32_t*>(&y);
+              for (int j = 0; j < kCols; ++j) x[j] = skinny_silu(x[j]) * u[j];
             }
-          } else {
+            uint32_t w[kCols / 2];
+            if (bf16) {
 #pragma unroll
-            for (int j = 0; j < kCols / 2; ++j) {
-              __half2 y = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
-              w[j] = *reinterpret_cast<uint32_t*>(&y);
+              for (int j = 0; j < kCols / 2; ++j) {
+                __nv_bfloat162 y = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+                w[j] = *reinterpret_cast<uint32_t*>(&y);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < kCols / 2; ++j) {
+                __half2 y = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
+                w[j] = *reinterpret_cast<uint32_t*>(&y);
+              }
             }
-          }
-          if (row_ok) {
-            uint8_t* const dst = c_row + static_cast<int64_t>(g_lo + g) * 16;
+            if (row_ok) {
+              uint8_t* const dst = c_row + static_cast<int64_t>(g_lo + g) * 16;
 #pragma unroll
-            for (int k = 0; k < kCols / 8; ++k) st_global_v4(dst + k * 16, make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
+              for (int k = 0; k < kCols / 8; ++k) st_global_v4(dst + k * 16, make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
+            }
+          };
+          int g = lo;
+          for (float x[16], u[16]; g + 2 <= hi; g += 2) finish(g, x, u);
+          if (g < hi) {
+            float x[8], u[8];
+            finish(g, x, u);
           }
-        };
-        int g = lo;
-        for (float x[16], u[16]; g + 2 <= hi; g += 2) finish(g, x, u);
-        if (g < hi) {
-          float x[8], u[8];
-          finish(g, x, u);
         }
       }
       tc_fence_before_sync();

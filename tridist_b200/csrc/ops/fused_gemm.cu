@@ -197,6 +197,7 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
     us = std::max(us, dram) + t.fixed;
     if (best_us >= 0 && us >= best_us) continue;
     best_us = us;
+    best.tile_us = us;
     best.bn = t.bn;
     best.allow_pair = t.pairs;
     best.allow_wide = t.blocks == 4 ? 1 : 0;
@@ -544,10 +545,13 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
     p.env.rank = static_cast<uint32_t>(d.rank);
   }
   plan->grid_x = grid_for(d, plan->prm[0], d.max_ctas, num_sms());
-  if (d.few_rows && d.R == 1 && d.M <= 128 && d.prof == 0 && d.c % 16 == 0 && d.ldc % 8 == 0) {
-    plan->skinny = true;
+  if (d.few_rows && d.R == 1 && d.M <= 256 && d.prof == 0 && d.c % 16 == 0 && d.ldc % 8 == 0) {
     SkinnyParams& f = plan->few;
     f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, num_sms());
+    plan->skinny = d.M <= 128 || d.few_rows == 2 || f.us < d.tile_us;
+  }
+  if (plan->skinny) {
+    SkinnyParams& f = plan->few;
     if (f.swiglu) f.up_row0 = d.swiglu_up_row0;
     f.tma_a = make_tmap(reinterpret_cast<void*>(d.a), d.a_rows, d.K, d.lda, d.bf16, f.ar);
     f.tma_b = make_tmap(reinterpret_cast<void*>(d.b), d.b_rows, d.K, d.ldb, d.bf16, f.wr);

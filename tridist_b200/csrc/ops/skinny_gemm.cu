@@ -42,15 +42,19 @@ static SkinnyParams lay_out(int M, int N, int K, bool swiglu, bool bf16, int sms
   p.shares = std::min(rounds * can_run, ceil_div(p.groups, 2));
   p.share = even_runs(p.groups, p.shares);
   p.workers = std::min(p.shares, can_run);
+  p.mb = ceil_div(M, 128);
   p.ar = up_to(M, 8);
   p.wr = 8 * (p.share.len + (p.share.more > 0 ? 1 : 0));
   p.nb = up_to(p.wr, 16);
   p.mma_n = p.boxes * p.nb;
   p.own = ceil_div(p.wr / 8, cluster);
   p.warps = ceil_div(M, 32);
-  const int xbuf = (cluster - 1) * p.boxes * p.own * p.warps * 1024;
+  const int parts = (cluster - 1) * p.boxes * p.own * p.warps * 1024;
+  // (two blocks' parts would take two stages of the ring from it)
+  p.parts_in_ring = (cluster > 1 && p.mb == 2) ? 1 : 0;
+  const int xbuf = p.parts_in_ring ? 0 : parts;
   const int block = (p.ar + p.nb * p.boxes) * 128;
-  p.pad = (128 - p.ar) * 128;
+  p.pad = (128 * p.mb - p.ar) * 128;
   const int room = kSkinnySmem - p.pad - xbuf;
   const int range = p.range.len + (p.range.more > 0 ? 1 : 0);
   p.kw = 8;
@@ -58,14 +62,14 @@ static SkinnyParams lay_out(int M, int N, int K, bool swiglu, bool bf16, int sms
   p.stage_bytes = p.kw * block;
   p.stages = std::min(kSkinnyMaxStages, room / p.stage_bytes);
   p.stages = std::max(1, std::min(p.stages, ceil_div(range, p.kw) * ceil_div(p.shares, p.workers)));
-  p.smem_bytes = p.stages * p.stage_bytes + p.pad + xbuf;
+  p.smem_bytes = std::max(p.stages * p.stage_bytes + p.pad + xbuf, parts);
   p.acc_cols = up_to(p.mma_n, 32);
   const int bufs = p.shares > p.workers ? 2 : 1;
   // runs of 16 k-blocks or more, four of them over the whole of K
-  while (2 << p.accs_log2 <= 4 / cluster && (bufs * p.acc_cols << (p.accs_log2 + 1)) <= 512 &&
+  while (2 << p.accs_log2 <= 4 / cluster && (p.mb * bufs * p.acc_cols << (p.accs_log2 + 1)) <= 512 &&
          (32 << p.accs_log2) <= p.range.len) ++p.accs_log2;
   p.tmem_cols = 32;
-  while (p.tmem_cols < bufs * p.acc_cols << p.accs_log2) p.tmem_cols *= 2;
+  while (p.tmem_cols < p.mb * bufs * p.acc_cols << p.accs_log2) p.tmem_cols *= 2;
   return p;
 }
 
@@ -79,18 +83,24 @@ SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms) {
   double best_us = -1;
   for (int cl2 = 0; 1 << cl2 <= kSkinnyMaxCluster; ++cl2)
     for (int most = 128; most <= 256; most *= 2) {
-      const SkinnyParams p = lay_out(M, N, K, swiglu, bf16, sms, cl2, most);
+      SkinnyParams p = lay_out(M, N, K, swiglu, bf16, sms, cl2, most);
+      if (best_us >= 0 && (p.tmem_cols > 512 || p.smem_bytes > kSkinnySmem)) continue;
       if (cl2 > 0 && (p.range.len < 2 || p.shares > p.workers)) continue;     // (a cluster meets once)
       if (best_us >= 0 && p.stages * p.stage_bytes < 120 * 1024) continue;    // (too little in flight)
+      const double mma = p.mb * 4 * std::max(p.mma_n, 48) / 2 / 1.7e3;        // us a k-block
       const double rounds = ceil_div(p.shares, p.workers);
       const double dram = static_cast<double>(N) * p.boxes * K * 2 / 6.3e6;
-      const double cta = rounds * (p.range.len + 1) * std::max((p.ar + p.wr * p.boxes) * 128 / 0.12e6, 0.13);
-      const double us = std::max(dram, cta) + 0.3 * std::min(dram, cta) + (cl2 == 0 ? 0.0 : cl2 == 1 ? 2.5 : 5.0);
+      const double cta = rounds * (p.range.len + 1) * std::max({(p.ar + p.wr * p.boxes) * 128 / 0.12e6, mma, 0.13});
+      const double us = std::max(dram, cta) + 0.3 * std::min(dram, cta) + (cl2 == 0 ? 0.0 : cl2 == 1 ? 2.5 : p.mb == 1 ? 5.0 : 9.0);
       if (best_us < 0 || us < 0.98 * best_us) {
         best = p;
         best_us = us;
       }
     }
+  // With start and epilogue. Two blocks of A leave the ring three to five short stages: 12 % more. The tiles of the general
+  // kernel are faster where they fill the device with a long K to cut. us here and there: 192 x 896 x 608 8.9 and 14.3,
+  // 256 x 11008 x 4096 45 and 67, 192 x 29568 x 8192 109 and 132; 192 x 8192 x 28672 120 and 111.
+  best.us = (best_us + 4.0) * (best.mb == 2 ? 1.12 : 1.0);
   return best;
 }
 

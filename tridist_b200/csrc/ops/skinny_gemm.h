@@ -1,4 +1,4 @@
-// C = A @ B^T for at most 128 rows of A on one rank: how the work is laid out, and its launch.
+// C = A @ B^T for at most 256 rows of A on one rank: how the work is laid out, and its launch.
 #pragma once
 #include <cuda.h>
 
@@ -35,17 +35,20 @@ struct SkinnyParams {
   int32_t shares;          // runs of groups, dealt round-robin to the workers
   EvenRuns share, range;   // groups of the shares, k-blocks of the ranges
   int32_t workers;
+  int32_t mb;              // 128-row blocks of A
   int32_t ar;              // rows of A in shared memory
   int32_t wr, nb, boxes;   // rows of B per box, rows of shared memory per box, boxes per k-block (SwiGLU: gate, up)
   int32_t kw;              // k-blocks per stage
   int32_t stages, stage_bytes;
-  int32_t pad;             // bytes behind the ring: the MMA reads 128 rows of A, whatever their number
+  int32_t pad;             // bytes behind the ring: the MMA reads whole blocks of A, whatever the number of rows
   int32_t mma_n;           // columns of the MMA
   int32_t accs_log2, acc_cols;   // accumulators a CTA's K sum is spread over, tensor memory columns of each
   int32_t tmem_cols;
   int32_t own;             // most groups of a share that one CTA of the cluster sums up
-  int32_t warps;           // epilogue warps with rows
+  int32_t warps;           // 32-row quarters of the blocks that have rows
+  int32_t parts_in_ring;   // the CTAs of a cluster exchange parts in the ring, when it has been read
   int32_t smem_bytes;
+  double us;               // expected time
   void* c;
   int64_t ldc;
   WaitEnv env;

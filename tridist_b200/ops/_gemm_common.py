@@ -223,7 +223,7 @@ def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr:
              allow_wide=env_int("TRIDIST_WIDE", 1), allow_splitk=env_int("TRIDIST_SPLITK", 1),
              # (ranks that compute together keep the tiles their exchange was measured with)
              by_rounds=1 if R == 1 else 0,
-             few_rows=1 if (free and M <= 128) else 0, fit_tile=1 if free else 0,
+             few_rows=1 if (free and M <= 256) else 0, fit_tile=1 if free else 0,
              raster_g=env_int("TRIDIST_RASTER_G", 0),
              l2_ahead=env_int("TRIDIST_L2_AHEAD", 0),
              prof=(prof_buffer().data_ptr() if prof_buffer() is not None else 0),
