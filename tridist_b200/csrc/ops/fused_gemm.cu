@@ -167,7 +167,10 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
 
 // Local launches: which of the four tiles, by the time expected of it. A round of tiles takes so many us a
 // k-block, a cut last round its share of them and the parking and adding of the partials, 512 x 256 tiles their
-// epilogue in every round (both accumulators are in use), any of them no less than the operands take from DRAM.
+// epilogue in every round (both accumulators are in use), any of them no less than the operands take from DRAM, nor
+// than the product takes under the power cap: at 1.25 PFLOP/s in long runs by 512 x 256 tiles, the slower the more
+// operands a tile moves per FLOP (fp16, 2560 x 13312 x 16384 927 us as 512 x 256 tiles and 962 as 256 x 256, which
+// need less of a last round).
 // The constants are fitted to 64 shapes of 192 to 8192 rows, each of the tiles timed in turn (the tile chosen was 0.6 %
 // slower than the fastest on average, 7 % with the rule by rounds alone), but for 4 % more on 256 x 256 tiles: in
 // long runs under the power cap their operand traffic costs that much. us with 128 x 128, 128 x 256, 256 x 256 and 512 x 256
@@ -175,14 +178,15 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
 // 4096 485, 316, 276, 314; 1728 x 12288 x 12288 656, 416, 370, 446; 8192 x 6144 x 12288 774 as 512 x 256, 800 as 256 x 256.
 static GemmPlanDesc fit_tile(GemmPlanDesc d) {
   if (!d.fit_tile || d.R != 1 || d.sched != SCHED_NATURAL || d.max_ctas > 0 || d.probe != 0) return d;
-  struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi; };
+  struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi, energy; };
   const bool swiglu = d.epi == EPI_SWIGLU;
-  const Tile tiles[4] = {{128, 1, 0, 0.375, 8.0, 5.0, 0.0},
-                         {256, 1, 0, 0.47, 10.0, 6.5, 0.0},
-                         {256, 2, 1, 0.42, 12.0, 6.0, 0.0},
-                         {256, 4, 1, 0.78, 12.0, 12.0, swiglu ? 6.0 : 3.5}};
+  const Tile tiles[4] = {{128, 1, 0, 0.375, 8.0, 5.0, 0.0, 1.45},
+                         {256, 1, 0, 0.47, 10.0, 6.5, 0.0, 1.2},
+                         {256, 2, 1, 0.42, 12.0, 6.0, 0.0, 1.07},
+                         {256, 4, 1, 0.78, 12.0, 12.0, swiglu ? 6.0 : 3.5, 1.0}};
   const int mt = (d.M + BM - 1) / BM, kb = (d.K + BK - 1) / BK;
   const double dram = (static_cast<double>(d.N) * (swiglu ? 2 : 1) * d.K + static_cast<double>(d.M) * (d.K + d.N)) * 2 / 6.3e6;
+  const double power = 2.0 * d.M * d.N * (swiglu ? 2 : 1) * d.K / 1.25e9;
   double best_us = -1;
   GemmPlanDesc best = d;
   for (const Tile& t : tiles) {
@@ -194,7 +198,7 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
     const double whole = kb * t.per_kb;
     double us = static_cast<double>(n / g) * (whole + t.epi);
     if (left > 0) us += (s == 1 ? whole : std::min(whole, whole / s + t.meet)) + t.epi;
-    us = std::max(us, dram) + t.fixed;
+    us = std::max(std::max(us, dram) + t.fixed, power * t.energy);
     if (best_us >= 0 && us >= best_us) continue;
     best_us = us;
     best.tile_us = us;
