@@ -167,13 +167,6 @@ __device__ __forceinline__ uint4 ld_global_cg_v4(const void* p) {
                : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint4 ld_global_cg_v4_hint(const void* p, uint64_t policy) {
-  uint4 v;
-  asm volatile("ld.global.cg.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p), "l"(policy));
-  return v;
-}
 // Generic address: shared memory, or global memory that bypasses L1.
 __device__ __forceinline__ uint4 ld_cg_v4(const void* p) {
   uint4 v;

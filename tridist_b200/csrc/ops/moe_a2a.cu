@@ -389,8 +389,9 @@ moe_dispatch_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restric
 // A whole 8 KB row is one request and a full stage keeps 64 KB in flight whatever the look-ups take,
 // where scattered reads of 2 KB are what DRAM serves slowly: 20 011 tokens of 8 KB rows, topk 8, 237 us,
 // 6.2 TB/s. A row is read once, so its lines are the first to leave L2 again and what dispatch or the experts
-// left there stays until it is read: 4096 tokens of 8 KB, topk 8, a round 118 us without, 112 with; by registers, 16384
-// tokens of 4 KB, topk 8, 286 us without, 276 with. A stage that is not full is wasted: 24 KB in flight at topk 1 (see launch_combine).
+// left there stays until it is read: 4096 tokens of 8 KB, topk 8, a round 115 us without, 108.5 with. (The same on the
+// register form's loads: 8192 tokens of 8 KB, topk 4, 128 and 125 us, but 9000 of 16 KB, topk 2, 166 and 170, 20000 of 8 KB,
+// topk 4, 299 and 304.) A stage that is not full is wasted: 24 KB in flight at topk 1 (see launch_combine).
 // ----------------------------------------------------------------------------
 template <bool kBf16>
 __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& v, float w) {
@@ -454,7 +455,6 @@ moe_combine_rows_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __res
   griddep_wait();
   if (d.R == 1) griddep_launch();
   if (d.R > 1 && !combine_ready(d, cta, tid)) return;
-  const uint64_t once = l2_evict_first();      // (a row is not read again)
   constexpr int kRows = 8 / V;            // expert rows whose pieces are loaded together
   const int64_t row_bytes = static_cast<int64_t>(d.H) * 2;
   const int n16 = static_cast<int>(row_bytes >> 4);
@@ -496,7 +496,7 @@ moe_combine_rows_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __res
         const bool have = j0 + b < topk && from != nullptr;
 #pragma unroll
         for (int u = 0; u < V; ++u)
-          v[b][u] = (have && i0 + 32 * u < n16) ? ld_global_cg_v4_hint(from + (static_cast<int64_t>(i0 + 32 * u) << 4), once)
+          v[b][u] = (have && i0 + 32 * u < n16) ? ld_global_cg_v4(from + (static_cast<int64_t>(i0 + 32 * u) << 4))
                                                 : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
