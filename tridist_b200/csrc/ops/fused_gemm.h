@@ -47,7 +47,7 @@ struct GemmPlanDesc {
   int few_rows = 0;     // one rank: the kernel of skinny_gemm.cuh for at most 128 rows, and for 256 where it is expected to be faster (2: for those too)
   double tile_us = 0;   // (the time that fit_tile expects)
   int fit_tile = 0;     // bn, pairs and the tile's height by the time expected of them (one rank; see fit_tile)
-  int by_rounds = 0;    // tile height by the rounds it takes (local launches; see choose_cta_mt)
+  int by_rounds = 0;    // tile height by the rounds it takes (local launches whose width is given; see choose_cta_mt)
   int raster_g = 0;     // row units walked together (0 = sized so that their A rows stay in L2)
   int l2_ahead = 0;      // k-blocks of L2 look-ahead of the operand loads (0 = none)
   // all-gather

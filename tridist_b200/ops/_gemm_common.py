@@ -36,7 +36,8 @@ def choose_bn(M: int, N: int, swiglu: bool = False, K: int = 0, local: bool = Fa
     through the L2 fabric, which is what bounds that shape.
 
     ``local`` (one rank): 256 as well where the K split of the CTA pairs' tiles fills three quarters
-    of the 74 pairs (256 rows, K 8192, N 8192: 47 us on 64 pairs, 74 us on 128 tiles of 128 x 128)."""
+    of the 74 pairs (256 rows, K 8192, N 8192: 47 us on 64 pairs, 74 us on 128 tiles of 128 x 128). A plan that may
+    pick its tile itself (``fit_tile`` of the descriptor) takes this width only as part of its key."""
     if swiglu:
         return 256       # gate and up halves are two 128-row TMA boxes of one 256-wide tile
     forced = env_int("TRIDIST_FORCE_BN", 0)
