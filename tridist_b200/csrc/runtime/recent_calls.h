@@ -29,7 +29,7 @@ class RecentCalls {
     gemm_plan_launch(it->second.plan, round, static_cast<int>(round & 1u), 0, 0, stream);
     return true;
   }
-  void remember(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, int64_t plan, py::object cache_key) {
+  void remember(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, int64_t plan, pybind11::object cache_key) {
     Key k;
     if (!width_forced() && key_of(a, b, c, tag, k)) calls_[k] = Call{plan, 0, std::move(cache_key)};
   }
@@ -38,12 +38,12 @@ class RecentCalls {
   }
   void clear() { calls_.clear(); }
   // Keys of the plans launched from here since the last time, the least recent first.
-  std::vector<py::object> drain() {
+  std::vector<pybind11::object> drain() {
     std::vector<Call*> v;
     for (auto& c : calls_)
       if (c.second.used > 0) v.push_back(&c.second);
     std::sort(v.begin(), v.end(), [](const Call* x, const Call* y) { return x->used < y->used; });
-    std::vector<py::object> out;
+    std::vector<pybind11::object> out;
     for (Call* c : v) {
       out.push_back(c->cache_key);
       c->used = 0;
@@ -72,7 +72,7 @@ class RecentCalls {
   struct Call {
     int64_t plan;
     uint64_t used;
-    py::object cache_key;
+    pybind11::object cache_key;
   };
   static bool key_of(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, Key& k) {
     int i = 0;
