@@ -48,3 +48,35 @@ def test_repeated_experts_and_rows_past_the_end(T):
         else:
             w.check()
         finalize_moe_a2a_context(ctx)
+
+
+@pytest.mark.parametrize("T", [24, 64, 400])
+def test_tokens_written_by_the_kernel_in_front(T):
+    """A GEMM, or the combine of the round before, writes the tokens right in front of a small dispatch, over inputs
+    that change from round to round in the same buffers."""
+    import test_gpu_ops
+    from tridist_b200.ops import (create_moe_a2a_intra_node_context, finalize_moe_a2a_context,
+                                  moe_combine_intra_node_op, moe_dispatch_intra_node_op)
+    from tridist_b200.ops._gemm_common import gemm_nt
+    w = test_gpu_ops._world1()
+    E, H, topk, K, dt = 16, 4096, 4, 512, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ctx = create_moe_a2a_intra_node_context(E, H, dt, T, topk, 0, 1, BLOCK_H=H, world=w)
+    b = (torch.randn((H, K), generator=g, device="cuda") * 0.05).to(dt)
+    tokens = torch.empty((T, H), dtype=dt, device="cuda")
+    of = torch.arange(T, device="cuda").repeat_interleave(topk)
+    for _ in range(8):
+        x = torch.randn((T, K), generator=g, device="cuda").to(dt)
+        idx = torch.randint(0, E, (T, topk), generator=g, device="cuda", dtype=torch.int32)
+        gemm_nt(x, b, out=tokens)
+        moe_dispatch_intra_node_op(tokens, idx, ctx)
+        sc = ctx.scatter_idx.flatten().long()
+        got = ctx.recv[sc]
+        assert torch.equal(got, tokens[of])
+        ctx.out[sc] = got + 1
+        idx2 = torch.randint(0, E, (T, topk), generator=g, device="cuda", dtype=torch.int32)
+        moe_combine_intra_node_op(ctx, idx, tokens)
+        moe_dispatch_intra_node_op(tokens, idx2, ctx)
+        assert torch.equal(ctx.recv[ctx.scatter_idx.flatten().long()], tokens[of])
+    w.check()
+    finalize_moe_a2a_context(ctx)

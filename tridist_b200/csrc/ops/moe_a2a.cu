@@ -190,7 +190,10 @@ constexpr int kRowThreads = 128;
 // Metadata and dispatch of one rank's small batch in one kernel: every CTA counts ALL the pairs, and those in
 // front of its own tokens, in shared memory, so that no CTA waits for another and a pair's slot is its place among
 // the pairs of its expert. Bound by latency: the pairs' load, the counts, the prefix sum and the rows' stores follow
-// one another once, where two kernels did so twice (64 tokens of 8 KB, topk 8: 7.2 us a round against 10.0). CTA (c, s) then stores slice s of the rows of tokens [c * per, (c + 1) * per).
+// one another once, where two kernels did so twice (64 tokens of 8 KB, topk 8: 7.2 us a round against 10.0). CTA (c, s)
+// then stores slice s of the rows of tokens [c * per, (c + 1) * per). It is the first kernel of a round, launched while
+// the GEMM or combine in front of it still writes the tokens: they are not read past the coherent path, which wants data
+// that nobody writes while the kernel lives. (moe_dispatch_kernel stands behind the metadata kernel and may.)
 constexpr int kRouteThreads = 256;
 
 __global__ void __launch_bounds__(kRouteThreads)
@@ -212,7 +215,7 @@ moe_route_dispatch_kernel(const __grid_constant__ MoeDesc d, int per, int slices
   const int i0 = slice * kRouteThreads + tid;      // this thread's first 16-byte piece of a row
   const uint8_t* const tokens = reinterpret_cast<const uint8_t*>(d.tokens) + (static_cast<int64_t>(i0) << 4);
   uint4 first = make_uint4(0u, 0u, 0u, 0u);        // (on its way while the pairs are counted)
-  if (t0 < t1 && i0 < n16) first = ld_global_nc_v4(tokens + t0 * row_bytes);
+  if (t0 < t1 && i0 < n16) first = ld_global_cg_v4(tokens + t0 * row_bytes);
   constexpr int kU = 8;                            // pairs of a thread whose loads are in flight together
   for (int b = tid; b < pairs; b += kU * kRouteThreads) {
     int e[kU];
@@ -289,7 +292,7 @@ moe_route_dispatch_kernel(const __grid_constant__ MoeDesc d, int per, int slices
     const int32_t* const rows = own_row + (t - t0) * topk;
     int64_t off = 0;
     for (int i = i0; i < n16; i += slices * kRouteThreads, off += step) {
-      const uint4 v = (t == t0 && off == 0) ? first : ld_global_nc_v4(tokens + t * row_bytes + off);
+      const uint4 v = (t == t0 && off == 0) ? first : ld_global_cg_v4(tokens + t * row_bytes + off);
 #pragma unroll 4
       for (int j = 0; j < topk; ++j) {
         const int r = rows[j];
