@@ -155,3 +155,34 @@ def test_two_blocks_of_rows(M, N, K, swiglu, cluster, monkeypatch):
             bound = (exact.abs() * (2.0 ** -11 if dt == torch.float16 else 2.0 ** -8) * 1.01 + exact.abs() * 2.0 ** -18 +
                      1.1 * e[:, :N] * up.abs() + F.silu(gate).abs() * e[:, N:] + 2.0 ** -24)
         assert bool(((out.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 4096, 1376), (128, 8192, 28672), (64, 2048, 16384), (256, 11008, 4096)])
+def test_few_rows_that_give_up_leave_the_context_usable(M, N, K):
+    """With the abort word raised every role leaves the first wait that looks at it, whatever the others still have on
+    their way: the call reports it or is complete, and the calls after it are right."""
+    from tridist_b200.ops import create_gemm_ar_intra_node_context, finalize_gemm_ar_context, gemm_ar_intra_node_op
+    from tridist_b200.parallel.runtime import ProcessWorld, native
+    C, w, dt = native(), ProcessWorld(0, 1), torch.bfloat16
+    ctx = create_gemm_ar_intra_node_context(M, N, dt, dt, 0, 1, M_PER_CHUNK=64, world=w)
+    a, b = _rand((M, K), 11, dt), _rand((N, K), 12, dt)
+    c = torch.empty((M, N), dtype=dt, device="cuda")
+    gemm_ar_intra_node_op(a, b, c, ctx)
+    torch.cuda.synchronize()
+    w.check()
+    ref = c.clone()
+    exact = a.double() @ b.double().t()
+    assert bool(((ref.double() - exact).abs() <= _bound(a, b, exact, dt)).all())
+    for _ in range(5):
+        c.zero_()
+        C.fill_u32(w.abort_word, 1, 5)
+        gemm_ar_intra_node_op(a, b, c, ctx)
+        torch.cuda.synchronize()
+        assert w.status()[0] == 5 or torch.equal(c, ref)
+        w.clear_status()
+        for _ in range(2):
+            gemm_ar_intra_node_op(a, b, c, ctx)
+        torch.cuda.synchronize()
+        w.check()
+        assert torch.equal(c, ref)
+    finalize_gemm_ar_context(ctx)

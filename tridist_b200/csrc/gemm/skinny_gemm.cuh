@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
     griddep_wait();
     griddep_launch();
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, armed = 0;                // armed: stages that a load was asked for
     bool ok = true;
     for (int v = worker; ok && v < shares; v += workers) {
       const int b_row = share.start(v) * 8;
@@ -122,14 +122,24 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
           }
         }
         __syncwarp();
+        armed |= 1u << stage;
         if (++stage == stages) { stage = 0; phase ^= 1u; }
       }
     }
-    if (!ok && lane == 0) {
-      // gave up: the loads in flight land before the shared memory goes. (No barrier counts them alone: the
-      // other loader may have left its half of a stage out. They take microseconds.)
-      const uint64_t t0 = globaltimer_ns();
-      while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    if (lane == 0) {
+      // The loads in flight land before the shared memory goes, whoever else has given up: a loader that is through has
+      // up to a ring of them on their way, which nobody but the MMA warp would wait for.
+      if (!ok) {
+        // (no barrier counts these alone: the other loader may have left its half of a stage out; they take microseconds)
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+      } else if (warp == 0) {
+        WaitEnv quiet{};                          // no status, no abort word: this wait only drains
+        quiet.rank = env.rank;
+        quiet.timeout_ns = 2000000ull;
+        for (int s = 0; s < stages; ++s)
+          if ((armed >> s & 1u) != 0u && !wait_mbar(&full_bar[s], s < stage ? phase : phase ^ 1u, quiet, SITE_PIPE_FULL, s)) break;
+      }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -199,8 +209,9 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
       if (lead) umma_commit(&acc_full[buf]);
       __syncwarp();
     }
-    if (!ok && lead) {
-      // gave up: the MMAs already issued must retire before the tensor memory is freed
+    if (lead) {
+      // The MMAs issued retire before tensor and shared memory go, also where the warps that wait for their sums
+      // have given up.
       umma_commit(&drain_bar);
       WaitEnv quiet{};
       quiet.rank = env.rank;
