@@ -1020,18 +1020,22 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         prof[PROF_LOAD_FLAG_WAIT] = acc_a;
         prof[PROF_LOAD_EMPTY_WAIT] = acc_b;
       }
-      if (!ok) {
-        // Unwinding: let the loads already issued land before the CTA's shared
-        // memory is released (each such wait is itself bounded).
-        for (int s = 0; s < TS::kStages; ++s) {
-          if (!((pending >> s) & 1u)) continue;
-          // the stage was armed in the most recent pass over slot s
-          const uint32_t par = (s < static_cast<int>(stage)) ? phase : (phase ^ 1u);
-          WaitEnv quiet{};                 // no status, no abort words: this wait only drains
-          quiet.rank = env.rank;
-          quiet.timeout_ns = 2000000ull;   // loads land within microseconds; never linger here
-          if (leader) wait_mbar(&full_bar[s], par, quiet, SITE_PIPE_FULL, s);
-        }
+      // The loads issued land before the CTA's shared memory is released, whoever else has given up: this warp may be
+      // through with up to a ring of them on their way, which only the MMA warp would wait for. (The leader's barriers
+      // count the loads of both CTAs of a pair, and the pair leaves together.)
+      for (int s = 0; leader && s < TS::kStages; ++s) {
+        if (!((pending >> s) & 1u)) continue;
+        // the stage was armed in the most recent pass over slot s
+        const uint32_t par = (s < static_cast<int>(stage)) ? phase : (phase ^ 1u);
+        WaitEnv quiet{};                 // no status, no abort words: this wait only drains
+        quiet.rank = env.rank;
+        quiet.timeout_ns = 2000000ull;   // loads land within microseconds; never linger here
+        if (!wait_mbar(&full_bar[s], par, quiet, SITE_PIPE_FULL, s)) break;
+      }
+      if (!ok && kCtaM == 2 && lead) {
+        // (the other CTA's half of these stages may never come, and no barrier counts this one's half alone)
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
       }
     }
   }
@@ -1197,8 +1201,8 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
         prof[PROF_MMA_FULL_WAIT] = acc_f;
         prof[PROF_MMA_TMEM_WAIT] = acc_t;
       }
-      if (!ok && lead) {
-        // Unwinding: MMAs already issued must retire before TMEM is freed.
+      if (lead) {
+        // MMAs already issued retire before TMEM is freed, also where the warps that wait for their sums have given up.
         if constexpr (kCtaM == 2) umma_commit_pair_local(drain_bar);
         else umma_commit(drain_bar);
         WaitEnv quiet{};
