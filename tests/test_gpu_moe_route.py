@@ -80,3 +80,32 @@ def test_tokens_written_by_the_kernel_in_front(T):
         assert torch.equal(ctx.recv[ctx.scatter_idx.flatten().long()], tokens[of])
     w.check()
     finalize_moe_a2a_context(ctx)
+
+
+def test_combine_that_gives_up_leaves_the_context_usable():
+    """With the abort word raised the ring's warps leave the first wait that looks at it, whatever copies are on their
+    way: the call reports it or is complete, and the rounds after it are right."""
+    from tridist_b200.ops import (create_moe_a2a_intra_node_context, finalize_moe_a2a_context,
+                                  moe_combine_intra_node_op, moe_dispatch_intra_node_op)
+    from tridist_b200.parallel.runtime import ProcessWorld, native
+    C, w = native(), ProcessWorld(0, 1)
+    T, E, H, topk, dt = 2048, 16, 4096, 8, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    tokens = torch.randn((T, H), generator=g, device="cuda").to(dt)
+    idx = torch.randint(0, E, (T, topk), generator=g, device="cuda", dtype=torch.int32)
+    ctx = create_moe_a2a_intra_node_context(E, H, dt, T, topk, 0, 1, BLOCK_H=H, world=w)
+    out = torch.empty_like(tokens)
+    for _ in range(5):
+        moe_dispatch_intra_node_op(tokens, idx, ctx)
+        ctx.out.copy_(ctx.recv)
+        out.zero_()
+        C.fill_u32(w.abort_word, 1, 5)
+        moe_combine_intra_node_op(ctx, idx, out)
+        torch.cuda.synchronize()
+        assert w.status()[0] == 5 or torch.equal(out, tokens * topk)
+        w.clear_status()
+        moe_combine_intra_node_op(ctx, idx, out)
+        torch.cuda.synchronize()
+        w.check()
+        assert torch.equal(out, tokens * topk)       # eight times a 16-bit number is exact
+    finalize_moe_a2a_context(ctx)

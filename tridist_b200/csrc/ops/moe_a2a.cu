@@ -575,19 +575,12 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
       }
     };
     if (items > 0) look_up();
-    for (int64_t k = 0; k < items; ++k) {
+    int64_t k = 0;
+    for (; k < items; ++k) {
       bool ok = true;
       if (lane == 0) ok = wait_mbar(&s_empty[slot], phase ^ 1u, d.env, SITE_PIPE_EMPTY, slot);
       ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
-      if (!ok) {
-        // gave up: let the copies in flight land before the shared memory goes (each wait bounded)
-        WaitEnv quiet{};
-        quiet.rank = d.env.rank;
-        quiet.timeout_ns = 2000000ull;
-        for (int s = 0; lane == 0 && s < kDepth && s < k; ++s)
-          wait_mbar(&s_full[s], s < slot ? phase : phase ^ 1u, quiet, SITE_PIPE_FULL, s);
-        return;
-      }
+      if (!ok) break;
       const uint8_t* src = expert_row(d, e, row, row_bytes, run == 0);
       const int64_t off = static_cast<int64_t>(run) * kRunBytes;
       const uint32_t have = __ballot_sync(0xFFFFFFFFu, src != nullptr);
@@ -602,6 +595,12 @@ moe_combine_kernel(const __grid_constant__ MoeDesc d0, const MoeDesc* __restrict
       if (++group == groups) { group = 0; unit += ncta; }
       if (k + 1 < items) look_up();
     }
+    // the copies in flight land before the shared memory goes, whoever has given up (each wait bounded)
+    WaitEnv quiet{};
+    quiet.rank = d.env.rank;
+    quiet.timeout_ns = 2000000ull;
+    for (int s = 0; lane == 0 && s < kDepth && s < k; ++s)
+      wait_mbar(&s_full[s], s < slot ? phase : phase ^ 1u, quiet, SITE_PIPE_FULL, s);
     return;
   }
 
