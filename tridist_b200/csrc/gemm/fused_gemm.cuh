@@ -1751,6 +1751,11 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
             }
           }
           tma_store_wait_all<0>();             // every byte of the part has been written
+          if (!ok) {
+            // gave up: the pieces on their way into the ring land before the shared memory goes (they take microseconds)
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+          }
         };
         // counts a finished part of chunk (row, ck) in; true for the thread that completes the chunk
         auto chunk_done = [&](int row, int ck) -> bool {
