@@ -117,3 +117,25 @@ def test_moe_refusals():
     exact = tokens.double() * wts.double().sum(1, keepdim=True)
     assert (out.double() - exact).norm() <= 2.0 ** -8 * exact.norm()
     finalize_moe_a2a_context(ctx)
+
+
+def test_width_forced_where_the_free_choice_starts_from_it(monkeypatch):
+    """A forced width of 256 and a free choice that has 256 in its key are two plans, natively remembered or not."""
+    from tridist_b200.ops import ag_gemm_intra_node_op, create_ag_gemm_intra_node_context, finalize_ag_gemm_context
+    w, dt, M, N, K = _world(), torch.bfloat16, 128, 4096, 512
+    ag = create_ag_gemm_intra_node_context(M, K, dt, dt, 0, 1, M_PER_CHUNK=128, world=w)
+    a, b = _rand((M, K), 1), _rand((N, K), 2)
+    h = torch.empty((M, N // 2), dtype=dt, device="cuda")
+    exact = a.double() @ b.double().t()
+    exact = torch.nn.functional.silu(exact[:, :N // 2]) * exact[:, N // 2:]
+    for i in range(3):
+        for forced in (False, True):
+            if forced:
+                monkeypatch.setenv("TRIDIST_FORCE_BN", "256")
+            else:
+                monkeypatch.delenv("TRIDIST_FORCE_BN", raising=False)
+            h.zero_()
+            ag_gemm_intra_node_op(a, b, h, ag, fuse_swiglu=True)
+            assert (h.double() - exact).norm() <= 2.0 ** -7 * exact.norm()
+    assert (ag.plans.misses, ag.plans.hits, ag.plans.recent.hits) == (2, 4, 2)
+    finalize_ag_gemm_context(ag)

@@ -23,7 +23,7 @@ class RecentCalls {
     if (!key_of(a, b, c, tag, k)) return false;
     auto it = calls_.find(k);
     if (it == calls_.end()) return false;
-    if (width_forced()) return false;
+    if (tile_forced()) return false;
     it->second.used = ++clock_;
     ++hits_;
     gemm_plan_launch(it->second.plan, round, static_cast<int>(round & 1u), 0, 0, stream);
@@ -31,7 +31,7 @@ class RecentCalls {
   }
   void remember(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, int64_t plan, pybind11::object cache_key) {
     Key k;
-    if (!width_forced() && key_of(a, b, c, tag, k)) calls_[k] = Call{plan, 0, std::move(cache_key)};
+    if (!tile_forced() && key_of(a, b, c, tag, k)) calls_[k] = Call{plan, 0, std::move(cache_key)};
   }
   void forget(int64_t plan) {
     for (auto it = calls_.begin(); it != calls_.end();) it = it->second.plan == plan ? calls_.erase(it) : std::next(it);
@@ -53,9 +53,12 @@ class RecentCalls {
   int64_t hits() const { return hits_; }
 
  private:
-  static bool width_forced() {      // by the environment, which the Python key looks at in every call
-    const char* v = std::getenv("TRIDIST_FORCE_BN");
-    return v != nullptr && *v != 0;
+  static bool tile_forced() {      // by the environment: the Python key, which such a call goes to, looks at it every time
+    for (const char* name : {"TRIDIST_FORCE_BN", "TRIDIST_MAX_CTAS"}) {
+      const char* v = std::getenv(name);
+      if (v != nullptr && *v != 0) return true;
+    }
+    return false;
   }
   static constexpr int kWords = 19;
   struct Key {

@@ -203,12 +203,17 @@ def read_prof(n_ctas: int = 148) -> Dict[str, Dict[str, float]]:
     return out
 
 
+def tile_is_free(world, R: int) -> bool:
+    """One rank: the tile (or, for few rows, the kernel) is the plan's own choice unless the environment makes it. Part
+    of every plan's key: a forced width may be the one that the free choice would start from."""
+    return (R == 1 and getattr(world, "kind", "") != "emulated" and not env_int("TRIDIST_MAX_CTAS", 0) and
+            not env_int("TRIDIST_FORCE_BN", 0))
+
+
 def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr: int, ldc: int,
               M: int, N: int, K: int, bn: int, op: int) -> Dict:
     assert a.stride(1) == 1 and b.stride(1) == 1, "operands must be row-major with unit inner stride"
-    # one rank: the tile (or, for few rows, the kernel) is the plan's own choice unless the environment makes it
-    free = (R == 1 and getattr(world, "kind", "") != "emulated" and not env_int("TRIDIST_MAX_CTAS", 0) and
-            not env_int("TRIDIST_FORCE_BN", 0))
+    free = tile_is_free(world, R)
     d = dict(op=op, epi=EPI_STORE, sched=SCHED_NATURAL, bn=bn, bf16=is_bf16(a.dtype), rank=rank, R=R,
              M=M, N=N, K=K, a=a.data_ptr(), a_rows=a.shape[0], lda=a.stride(0),
              b=b.data_ptr(), b_rows=b.shape[0], ldb=b.stride(0), c=c_ptr, ldc=ldc,
@@ -298,10 +303,10 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     assert out.stride(1) == 1
-    free = bn is None and local and not max_ctas and not probe      # (the tile is nobody's choice)
+    w = plain_world()
+    free = bn is None and local and not max_ctas and not probe and tile_is_free(w, 1)      # (the tile is nobody's choice)
     if bn is None:
         bn = choose_bn(M, N, swiglu, K=K, local=local and not max_ctas)    # (the rule counts on all SMs)
-    w = plain_world()
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
            out.stride(0), bn, swiglu, a.dtype, max_ctas, probe, local, free)
 

@@ -40,7 +40,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, EPI_SWIGLU, OP_AG, SCHED_NATURAL, SCHED_SEGMENT, PlanCache,
-                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes)
+                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
 
 _CONSUMER_BLOCK_M = 128
 _CONSUMER_BLOCK_N = 128
@@ -254,7 +254,7 @@ def _plan(ctx, a, b, c, swiglu=False):
     key = (a.data_ptr(), b.data_ptr(), c.data_ptr(), m_pr, n_rows, K, a.stride(0), b.stride(0), c.stride(0),
            a.dtype, swiglu, bn, tuple(order), baked_table.data_ptr() if baked_table is not None else 0,
            ctx.observe, getattr(ctx, "emu_table_header", False), getattr(ctx, "seg_bands", 0), getattr(ctx, "seg_own_first", 0), ctx.transport,
-           ctx.push_ctas)
+           ctx.push_ctas, tile_is_free(ctx.world, R))
 
     def make():
         d = base_desc(ctx.world, rank, R, a, b, c.data_ptr(), c.stride(0), M, N, K, bn, OP_AG)

@@ -45,7 +45,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, OP_AR1, OP_AR2, OP_PLAIN, SCHED_STRIDED, PlanCache,
-                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes)
+                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
 
 
 @dataclass
@@ -187,7 +187,7 @@ def _plan(ctx, a, b, c, mode, parity):
             (ctx.mc.local_ptr + (2 + parity) * plane)
         res_is_c = 1 if (c.data_ptr() == res_ptr and c.stride(0) == N) else 0
     key = (a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, a.stride(0), b.stride(0), c.stride(0),
-           a.dtype, bn, mode, res_is_c, parity if res_is_c else -1)
+           a.dtype, bn, mode, res_is_c, parity if res_is_c else -1, tile_is_free(ctx.world, R))
 
     def make():
         op = {"local": OP_PLAIN, "gemm": OP_PLAIN, "one_shot": OP_AR1, "two_shot": OP_AR2,

@@ -36,7 +36,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, OP_RS, SCHED_NATURAL, SCHED_SEGMENT, PlanCache, base_desc, choose_bn,
-                           debug_check, rotation_order, tensor_extent_bytes)
+                           debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
 
 
 @dataclass
@@ -158,7 +158,7 @@ def _plan(ctx, a, b, out):
     # through the switch all ranks walk the same order (lockstep over the owners' segments)
     order = list(range(R)) if mode == "nvls" else (ctx.order_override or rotation_order(rank, R, 1, own_last=True))
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-           a.dtype, bn, tuple(order), mode, ctx.reduce_ctas, ctx.reduce_tail)
+           a.dtype, bn, tuple(order), mode, ctx.reduce_ctas, ctx.reduce_tail, tile_is_free(ctx.world, R))
 
     def make():
         d = base_desc(ctx.world, rank, R, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_RS)
