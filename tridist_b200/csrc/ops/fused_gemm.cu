@@ -210,6 +210,29 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
   return best;
 }
 
+// Whether launches of this plan go to the kernel of skinny_gemm.cuh, and its layout if they may. (That kernel walks all
+// tiles: a tile list stays with the general one.)
+static bool takes_few_rows(const GemmPlanDesc& d, int sms, SkinnyParams& f) {
+  if (!d.few_rows || d.R != 1 || d.sched != SCHED_NATURAL || d.M > 256 || d.prof != 0 || d.c % 16 != 0 || d.ldc % 8 != 0)
+    return false;
+  f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, sms);
+  return d.M <= 128 || d.few_rows == 2 || f.us < d.tile_us;
+}
+
+GemmChoice gemm_choice(const GemmPlanDesc& desc, int sms) {
+  const GemmPlanDesc d = fit_tile(desc);
+  SkinnyParams f;
+  std::memset(&f, 0, sizeof(f));
+  GemmChoice o;
+  o.few_rows = takes_few_rows(d, sms, f);
+  o.bn = d.bn;
+  o.cta_m = choose_cta_m(d);
+  o.row_blocks = choose_cta_mt(d, o.cta_m);
+  o.tile_us = d.tile_us;
+  o.few_rows_us = f.us;
+  return o;
+}
+
 // Everything the tile schedule depends on (shared by plan creation and the host-side dump).
 static void fill_schedule_fields(const GemmPlanDesc& d, int cta_m, int cta_mt, GemmParams& p) {
   const int bn_out = (d.epi == EPI_SWIGLU) ? d.bn / 2 : d.bn;
@@ -549,11 +572,7 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
     p.env.rank = static_cast<uint32_t>(d.rank);
   }
   plan->grid_x = grid_for(d, plan->prm[0], d.max_ctas, num_sms());
-  if (d.few_rows && d.R == 1 && d.M <= 256 && d.prof == 0 && d.c % 16 == 0 && d.ldc % 8 == 0) {
-    SkinnyParams& f = plan->few;
-    f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, num_sms());
-    plan->skinny = d.M <= 128 || d.few_rows == 2 || f.us < d.tile_us;
-  }
+  plan->skinny = takes_few_rows(d, num_sms(), plan->few);
   if (plan->skinny) {
     SkinnyParams& f = plan->few;
     if (f.swiglu) f.up_row0 = d.swiglu_up_row0;

@@ -87,6 +87,14 @@ struct GemmPlanDesc {
   uint32_t poll_ns = 0;   // pause between two polls of a cross-rank flag
 };
 
+// What runs for a descriptor, worked out on the host: the kernel, its tile, and the times expected where they were compared.
+struct GemmChoice {
+  bool few_rows = false;     // the kernel of skinny_gemm.cuh; the tile below is then that of calls it does not take
+  int bn = 0, cta_m = 1, row_blocks = 1;
+  double tile_us = 0, few_rows_us = 0;
+};
+GemmChoice gemm_choice(const GemmPlanDesc& d, int sms);
+
 int64_t gemm_plan_create(const GemmPlanDesc& d);
 void gemm_plan_destroy(int64_t id);
 // `order_table`: optional device int32[R] overriding the segment order for this call.
