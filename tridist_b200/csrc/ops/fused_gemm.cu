@@ -73,6 +73,7 @@ struct GemmPlan {
   int cta_mt;
   int grid_x;
   bool early_start;
+  bool staging;                       // of the tiles of one row block per CTA (taller ones always have it)
   bool skinny = false;                // few rows: launches go to the kernel of skinny_gemm.cuh
   SkinnyParams few;
   GemmParams* dev_params = nullptr;   // emulated multi-rank launches only
@@ -210,6 +211,17 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
   return best;
 }
 
+// Whether tiles leave through the staging area.
+static bool uses_staging(const GemmPlanDesc& d, int cta_m, int cta_mt) {
+  // operators that ship data to other ranks (epilogue tiles, all-gather push) need it
+  if (d.R > 1) return d.op == OP_RS || d.op == OP_AR1 || d.op == OP_AR2 || d.op == OP_AG;
+  // Local 256 x 256 tiles of a short K, whose epilogue shows, leave through it too; a long K rather has the seventh ring
+  // stage. us with and without (rows x N x K): 1984 x 8192 x 3696 108 and 118, 2048 x 9856 x 2656 89 and 101, 2432 x 4096
+  // x 1376 37 and 42; 2112 x 22016 x 4096 316 and 300, 8192 x 12288 x 6144 828 and 810. (Local launches only: the panel
+  // GEMMs of an operator of several ranks, which have neither mark, keep the ring that their exchange was measured with.)
+  return (d.fit_tile || d.by_rounds) && cta_m == 2 && cta_mt == 1 && (d.K + BK - 1) / BK < 60;
+}
+
 // Whether launches of this plan go to the kernel of skinny_gemm.cuh, and its layout if they may. (That kernel walks all
 // tiles: a tile list stays with the general one.)
 static bool takes_few_rows(const GemmPlanDesc& d, int sms, SkinnyParams& f) {
@@ -228,6 +240,7 @@ GemmChoice gemm_choice(const GemmPlanDesc& desc, int sms) {
   o.bn = d.bn;
   o.cta_m = choose_cta_m(d);
   o.row_blocks = choose_cta_mt(d, o.cta_m);
+  o.staging = uses_staging(d, o.cta_m, o.row_blocks);
   o.tile_us = d.tile_us;
   o.few_rows_us = f.us;
   return o;
@@ -498,6 +511,7 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
   plan->early_start = d.early_start && d.R == 1;
   plan->cta_m = choose_cta_m(d);
   plan->cta_mt = choose_cta_mt(d, plan->cta_m);
+  plan->staging = uses_staging(d, plan->cta_m, plan->cta_mt);
   for (int par = 0; par < 2; ++par) {
     GemmParams& p = plan->prm[par];
     std::memset(&p, 0, sizeof(p));
@@ -646,17 +660,8 @@ static int resident_ctas() {
   return cached;
 }
 
-static bool plan_uses_staging(const GemmParams& p) {
-  // operators that ship data to other ranks (epilogue tiles, all-gather push) need the staging area
-  // Local 256 x 256 tiles of a short K, whose epilogue shows, leave through it too; a long K rather has the seventh ring
-  // stage. us with and without (rows x N x K): 1984 x 8192 x 3696 108 and 118, 2048 x 9856 x 2656 89 and 101, 2432 x 4096
-  // x 1376 37 and 42; 2112 x 22016 x 4096 316 and 300, 8192 x 12288 x 6144 828 and 810.
-  if (p.R == 1 && p.cta_m == 2 && p.cta_mt == 1 && p.k_blocks < 60) return true;
-  return p.R > 1 && (p.op == OP_RS || p.op == OP_AR1 || p.op == OP_AR2 || p.op == OP_AG);
-}
-
 static int resident_ctas_of(const GemmPlan& plan) {
-  const bool st = plan_uses_staging(plan.prm[0]);
+  const bool st = plan.staging;
 #define TDB_RES(BN_, PAIR_, MT_)                                                            \
   (plan.bf16 ? (st ? resident_ctas<BN_, true, PAIR_, true, MT_>() : resident_ctas<BN_, true, PAIR_, (MT_ == 2), MT_>()) \
              : (st ? resident_ctas<BN_, false, PAIR_, true, MT_>() : resident_ctas<BN_, false, PAIR_, (MT_ == 2), MT_>()))
@@ -738,7 +743,7 @@ void gemm_plan_launch(int64_t id, uint32_t round, int parity, int64_t order_tabl
   p.comm_only = (flags >> 1) & 1;
   p.publish_only = (flags >> 2) & 1;
   const SplitScratch scratch = bind_sk_scratch(p, p.sk_tiles * p.sk_slices * p.cta_m, stream);
-  const bool staging = plan_uses_staging(p);
+  const bool staging = plan->staging;
 #define TDB_LAUNCH(BN_, PAIR_)                                                              \
   do {                                                                                      \
     if (plan->bf16) {                                                                       \

@@ -91,6 +91,7 @@ struct GemmPlanDesc {
 struct GemmChoice {
   bool few_rows = false;     // the kernel of skinny_gemm.cuh; the tile below is then that of calls it does not take
   int bn = 0, cta_m = 1, row_blocks = 1;
+  bool staging = false;      // (of tiles of one row block per CTA; taller ones always have it)
   double tile_us = 0, few_rows_us = 0;
 };
 GemmChoice gemm_choice(const GemmPlanDesc& d, int sms);
