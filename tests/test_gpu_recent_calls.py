@@ -139,3 +139,36 @@ def test_width_forced_where_the_free_choice_starts_from_it(monkeypatch):
             assert (h.double() - exact).norm() <= 2.0 ** -7 * exact.norm()
     assert (ag.plans.misses, ag.plans.hits, ag.plans.recent.hits) == (2, 4, 2)
     finalize_ag_gemm_context(ag)
+
+
+def test_moe_combine_refusals():
+    """What the combine kernels would read past the end of, or write in another type; and forms that stay accepted."""
+    from tridist_b200.ops import (create_moe_a2a_intra_node_context, finalize_moe_a2a_context,
+                                  moe_combine_intra_node_op, moe_dispatch_intra_node_op)
+    w, dt, T, E, H, topk = _world(), torch.bfloat16, 32, 8, 256, 2
+    ctx = create_moe_a2a_intra_node_context(E, H, dt, T, topk, 0, 1, BLOCK_H=H, world=w)
+    tokens = _rand((T, H), 1)
+    idx = torch.randint(0, E, (T, topk), device="cuda", dtype=torch.int32)
+    out, wts = torch.empty_like(tokens), torch.rand((T, topk), device="cuda")
+    for bad in [(tokens.cpu(), idx), (tokens, idx.cpu())]:
+        with pytest.raises(AssertionError):
+            moe_dispatch_intra_node_op(*bad, ctx)
+    moe_dispatch_intra_node_op(tokens, idx, ctx)
+    ctx.out[:] = ctx.recv
+    two = torch.cat([idx, idx])
+    for bad in [(idx.long(), out, wts), (idx[:, :1].contiguous(), out, wts), (idx[:1, :1].expand(T, topk), out, wts),
+                (idx.t().contiguous().t(), out, wts), (two, torch.cat([out, out]), None), (idx, out, wts[:, :1].contiguous()),
+                (idx, out, wts[:8]), (idx, out.float(), wts), (idx, out.half(), wts), (idx.cpu(), out, wts),
+                (idx, out.cpu(), wts), (idx, out, wts.cpu())]:
+        with pytest.raises(AssertionError):
+            moe_combine_intra_node_op(ctx, *bad)
+    exact = tokens.double() * wts.double().sum(1, keepdim=True)
+    for good in [(idx, out, wts), (idx, out, wts.flatten()), (idx.unsqueeze(-1), out, wts), (idx.cpu().pin_memory(), out, wts)]:
+        out.zero_()
+        moe_combine_intra_node_op(ctx, *good)
+        assert (out.double() - exact).norm() <= 2.0 ** -8 * exact.norm()
+    moe_dispatch_intra_node_op(tokens.cpu().pin_memory(), idx, ctx)
+    torch.cuda.synchronize()
+    w.check()
+    assert torch.equal(ctx.recv[ctx.scatter_idx.flatten().long()], tokens.repeat_interleave(topk, 0))
+    finalize_moe_a2a_context(ctx)

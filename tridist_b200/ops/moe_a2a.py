@@ -169,12 +169,30 @@ def _desc(ctx, tokens=None, topk_idx=None, output=None, topk_weights=None, T=0, 
     return d
 
 
+def _on_device(t) -> bool:
+    """Memory that a kernel can read: the device's own, or pinned host memory."""
+    return t.is_cuda or t.is_pinned()
+
+
 def _check_dispatch(tokens, topk_idx, ctx):
     T = tokens.shape[0]
     assert T <= ctx.max_tokens, "more tokens than the context was created for"
     assert tokens.shape[1] == ctx.hidden and tokens.is_contiguous() and tokens.dtype == ctx.input_dtype
     assert topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
     assert tuple(topk_idx.shape) == (T, ctx.topk)
+    assert _on_device(tokens) and _on_device(topk_idx), "tokens and topk_idx must be on the device"
+    return T
+
+
+def _check_combine(ctx, topk_idx, output, topk_weights):
+    T = topk_idx.shape[0]
+    assert T <= ctx.max_tokens, "more tokens than the context was created for"
+    assert topk_idx.dtype == torch.int32 and topk_idx.is_contiguous() and topk_idx.numel() == T * ctx.topk
+    assert tuple(output.shape) == (T, ctx.hidden) and output.is_contiguous() and output.dtype == ctx.input_dtype
+    assert _on_device(topk_idx) and _on_device(output), "topk_idx and output must be on the device"
+    if topk_weights is not None:
+        assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
+        assert topk_weights.numel() == T * ctx.topk and _on_device(topk_weights)
     return T
 
 
@@ -198,10 +216,7 @@ def moe_combine_intra_node_op(ctx, topk_idx, output, topk_weights=None):
     if isinstance(ctx.world, CpuWorld):
         return cpu_backend.moe_combine(ctx, topk_idx, output, topk_weights)
     if not (ctx._handle or _handle(ctx)).combine(ctx.meta_round, ctx.world.timeout_ns, topk_idx, topk_weights, output):
-        T = topk_idx.shape[0]
-        assert output.shape[0] == T and output.shape[1] == ctx.hidden and output.is_contiguous()
-        if topk_weights is not None:
-            assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
+        _check_combine(ctx, topk_idx, output, topk_weights)
         raise ValueError("tridist_b200: output and topk_weights do not fit the MoE context")
     return output
 
@@ -223,7 +238,8 @@ def moe_combine_emulated(ctxs, idx_list, out_list, w_list=None):
     ds = []
     for i, (ctx, idx, out) in enumerate(zip(ctxs, idx_list, out_list)):
         w = w_list[i] if w_list is not None else None
-        ds.append(_desc(ctx, topk_idx=idx, output=out, topk_weights=w, T=idx.shape[0]))
+        T = _check_combine(ctx, idx, out, w)
+        ds.append(_desc(ctx, topk_idx=idx, output=out, topk_weights=w, T=T))
     native().moe_emulated(ds, 2)
     return out_list
 
