@@ -39,3 +39,32 @@ def test_ranks_that_ship_tiles_have_the_staging_area():
 def test_given_width_of_a_local_launch():
     kw = dict(M=2048, N=8192, allow_wide=0, fit_tile=0, few_rows=0)
     assert _choice(K=3584, **kw)["staging"] and not _choice(K=4096, **kw)["staging"]
+
+
+@pytest.mark.parametrize("M,N,K,swiglu,few", [
+    (64, 10008, 20008, 0, False), (128, 3400, 21752, 1, False), (96, 4704, 14392, 1, False), (128, 20160, 24784, 1, False),
+    (16, 10008, 20008, 0, True), (64, 4096, 1376, 0, True), (96, 5352, 14576, 0, True), (128, 8192, 28672, 0, True),
+    (64, 712, 8680, 1, True), (128, 512, 22576, 1, True), (128, 2656, 37568, 1, True),
+    (256, 2736, 5720, 1, False), (192, 2240, 12616, 0, False),
+])
+def test_few_rows_by_the_alignment_of_the_rows(M, N, K, swiglu, few):
+    """At shapes whose times were measured; the general kernel then keeps the tile that it is given."""
+    from tridist_b200.ops._gemm_common import choose_bn
+    bn = choose_bn(M, N, bool(swiglu), K=K, local=True)
+    got = _choice(M=M, N=N, K=K, epi=swiglu, bn=bn)
+    assert got["few_rows"] == few
+    if not few:
+        assert got["bn"] == bn and got["cta_m"] == (2 if M > 128 and bn == 256 else 1)
+
+
+@pytest.mark.parametrize("part", ["a", "b", "lda", "ldb"])
+def test_alignment_is_that_of_addresses_and_strides(part):
+    kw = dict(M=64, N=10008, K=20032, a=1 << 20, b=1 << 30, lda=20032, ldb=20032)
+    assert _choice(**kw)["few_rows"]
+    kw[part] += 16 if part in "ab" else 8
+    assert not _choice(**kw)["few_rows"]
+
+
+def test_sizes_that_a_plan_refuses_are_not_laid_out():
+    for kw in (dict(M=64, N=0, K=64), dict(M=0, N=64, K=64), dict(M=64, N=64, K=0), dict(M=64, N=4, K=64)):
+        assert not _choice(**kw)["few_rows"]

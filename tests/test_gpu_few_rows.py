@@ -186,3 +186,41 @@ def test_few_rows_that_give_up_leave_the_context_usable(M, N, K):
         w.check()
         assert torch.equal(c, ref)
     finalize_gemm_ar_context(ctx)
+
+
+@pytest.mark.parametrize("M,N,K,swiglu", [
+    (33, 1000, 15016, False), (64, 4096, 1384, False), (100, 48, 8200, False), (128, 4704, 7192, True), (96, 3128, 48024, False),
+    (136, 2240, 12616, False), (200, 1256, 10024, True), (256, 520, 8008, False),
+])
+@pytest.mark.parametrize("few", [0, 1, 2])       # the general kernel, the rule's choice, the few-rows kernel
+def test_rows_on_odd_multiples_of_16_bytes(M, N, K, swiglu, few, monkeypatch):
+    from tridist_b200.ops import _gemm_common as common
+    from tridist_b200.ops._gemm_common import gemm_nt
+    from tridist_b200.parallel.runtime import native
+    C, dt = native(), torch.bfloat16
+    create, made = C.gemm_plan_create, []
+
+    def record(d):
+        d = dict(d, few_rows=few)
+        made.append(C.gemm_choice(d, 148)["few_rows"])
+        return create(d)
+
+    monkeypatch.setattr(C, "gemm_plan_create", record)
+    monkeypatch.setattr(common, "_plain_cache", common.PlanCache())      # (its key knows nothing of `few`)
+    a, b = _rand((M, K), 8, dt), _rand((2 * N if swiglu else N, K), 9, dt)
+    plane = torch.full((M + 1, N + 8), 7.0, dtype=dt, device="cuda")
+    out = plane[:M, :N]
+    gemm_nt(a, b, out=out, swiglu=swiglu)
+    gemm_nt(a, b, out=out, swiglu=swiglu)
+    torch.cuda.synchronize()
+    assert few == 1 or made == [few == 2]
+    assert bool((plane[M] == 7.0).all()) and bool((plane[:, N:] == 7.0).all())
+    exact = a.double() @ b.double().t()
+    bound = _bound(a, b, exact, dt)
+    if swiglu:
+        gate, up = exact[:, :N], exact[:, N:]
+        exact = F.silu(gate) * up
+        e = K * 2.0 ** -23 * (a.abs().double() @ b.abs().double().t())
+        bound = (exact.abs() * 2.0 ** -8 * 1.01 + exact.abs() * 2.0 ** -18 + 1.1 * e[:, :N] * up.abs() +
+                 F.silu(gate).abs() * e[:, N:] + 2.0 ** -24)
+    assert bool(((out.double() - exact).abs() <= bound).all())

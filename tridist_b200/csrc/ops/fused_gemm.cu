@@ -166,6 +166,12 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
   return 2;
 }
 
+// The largest power of two, up to 128, of whose bytes the rows of both operands start at multiples.
+static int row_alignment(const GemmPlanDesc& d) {
+  const int64_t bits = d.a | d.b | d.lda * 2 | d.ldb * 2 | 128;
+  return static_cast<int>(bits & -bits);
+}
+
 // Local launches: which of the four tiles, by the time expected of it. A round of tiles takes so many us a
 // k-block, a cut last round its share of them and the parking and adding of the partials, 512 x 256 tiles their
 // epilogue in every round (both accumulators are in use), any of them no less than the operands take from DRAM, nor
@@ -177,6 +183,9 @@ static int choose_cta_mt(const GemmPlanDesc& d, int cta_m) {
 // long runs under the power cap their operand traffic costs that much. us with 128 x 128, 128 x 256, 256 x 256 and 512 x 256
 // tiles (rows x N x K): 384 x 3328 x 1584 16.8, 23.6, 21.6, 25.2; 320 x 28672 x 8192 236, 160, 171, 171; 2112 x 22016 x
 // 4096 485, 316, 276, 314; 1728 x 12288 x 12288 656, 416, 370, 446; 8192 x 6144 x 12288 774 as 512 x 256, 800 as 256 x 256.
+// Rows on odd multiples of 16 bytes, which make every 128-byte piece of an operand lie in two lines, keep the given width and
+// the height by rounds: the constants were fitted without them, and the tiles they choose there move more operands (34
+// such shapes of 136 to 2000 rows: 1.7 % slower on average, up to 40 %).
 static GemmPlanDesc fit_tile(GemmPlanDesc d) {
   if (!d.fit_tile || d.R != 1 || d.sched != SCHED_NATURAL || d.max_ctas > 0 || d.probe != 0) return d;
   struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi, energy; };
@@ -203,6 +212,7 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
     if (best_us >= 0 && us >= best_us) continue;
     best_us = us;
     best.tile_us = us;
+    if (row_alignment(d) < 32) continue;
     best.bn = t.bn;
     best.allow_pair = t.pairs;
     best.allow_wide = t.blocks == 4 ? 1 : 0;
@@ -222,26 +232,52 @@ static bool uses_staging(const GemmPlanDesc& d, int cta_m, int cta_mt) {
   return (d.fit_tile || d.by_rounds) && cta_m == 2 && cta_mt == 1 && (d.K + BK - 1) / BK < 60;
 }
 
-// Whether launches of this plan go to the kernel of skinny_gemm.cuh, and its layout if they may. (That kernel walks all
-// tiles: a tile list stays with the general one.)
-static bool takes_few_rows(const GemmPlanDesc& d, int sms, SkinnyParams& f) {
-  if (!d.few_rows || d.R != 1 || d.sched != SCHED_NATURAL || d.M > 256 || d.prof != 0 || d.c % 16 != 0 || d.ldc % 8 != 0)
-    return false;
-  f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, sms);
-  return d.M <= 128 || d.few_rows == 2 || f.us < d.tile_us;
+// What a descriptor gets: the tile of the general kernel, and whether launches go to the kernel of skinny_gemm.cuh instead
+// (`few`, laid out in `f`). That kernel walks all tiles: a tile list stays with the general one.
+//
+// At most 128 rows go there. It was the faster kernel of 16 to 128 rows at 603 of 609 launches over weights of 8 MB to 2 GB
+// whose rows start on multiples of 64 bytes (0.40 to 1.0 of the other's time; the six, 128 rows of a K past 37000, took 2 to 14 %
+// more), and at all of 220 of 16 rows but for 5 % at one. Rows that start between cost its port, which re-reads A, more than
+// the general kernel's: there the expected times are compared, and the general kernel keeps the tile that it is given. us here and
+// there: 96 x 5352 x 14576 39.5 and 44.5, 128 x 2 x 20160 x 24784 with SwiGLU 438 and 391; on odd multiples of 16 bytes 64 x 10008
+// x 20008 109 and 90, 128 x 2 x 3400 x 21752 with SwiGLU 99 and 72. Up to 256 rows go there where it is expected to be faster.
+static GemmPlanDesc settle(const GemmPlanDesc& desc, int sms, bool& few, SkinnyParams& f) {
+  GemmPlanDesc d = fit_tile(desc);
+  few = false;
+  if (!d.few_rows || d.R != 1 || d.sched != SCHED_NATURAL || d.M < 1 || d.M > 256 || d.N < 8 || d.K < 8 || d.prof != 0 || d.c % 16 != 0 || d.ldc % 8 != 0)
+    return d;
+  const int align = row_alignment(d);
+  f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, sms, align < 32);
+  if (d.few_rows == 2 || d.M <= 32 || (d.M <= 128 && (align >= 64 || d.tile_us <= 0))) {
+    few = true;
+  } else if (d.M <= 128) {
+    few = f.us <= 1.1 * d.tile_us;
+    if (!few) {
+      d = desc;
+      d.fit_tile = d.few_rows = 0;
+    }
+  } else {
+    few = f.us < d.tile_us;
+  }
+  return d;
+}
+
+static GemmPlanDesc settle(const GemmPlanDesc& desc, int sms) {
+  bool few;
+  SkinnyParams f;
+  return settle(desc, sms, few, f);
 }
 
 GemmChoice gemm_choice(const GemmPlanDesc& desc, int sms) {
-  const GemmPlanDesc d = fit_tile(desc);
   SkinnyParams f;
   std::memset(&f, 0, sizeof(f));
   GemmChoice o;
-  o.few_rows = takes_few_rows(d, sms, f);
+  const GemmPlanDesc d = settle(desc, sms, o.few_rows, f);
   o.bn = d.bn;
   o.cta_m = choose_cta_m(d);
   o.row_blocks = choose_cta_mt(d, o.cta_m);
   o.staging = uses_staging(d, o.cta_m, o.row_blocks);
-  o.tile_us = d.tile_us;
+  o.tile_us = fit_tile(desc).tile_us;
   o.few_rows_us = f.us;
   return o;
 }
@@ -347,7 +383,7 @@ static SplitScratch bind_sk_scratch(GemmParams& p, int slots, cudaStream_t strea
 }
 
 std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& desc, int sms) {
-  const GemmPlanDesc d = fit_tile(desc);
+  const GemmPlanDesc d = settle(desc, sms);
   if (d.sched == SCHED_LIST) throw std::runtime_error("tridist_b200: a tile list is its own schedule");
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
@@ -375,7 +411,7 @@ std::vector<std::vector<std::array<int, 5>>> schedule_dump(const GemmPlanDesc& d
 // The K ranges of the tiles that are cut along K: {scheduling position, first CTA of the worker,
 // slice, slices, first k-block, end k-block} for every worker that takes part.
 std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& desc, int sms) {
-  const GemmPlanDesc d = fit_tile(desc);
+  const GemmPlanDesc d = settle(desc, sms);
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   const int cta_m = choose_cta_m(d);
@@ -393,7 +429,7 @@ std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& desc, int sms) {
 }
 
 std::vector<std::string> plan_check(const GemmPlanDesc& desc, const PlanExtents& e, int sms) {
-  const GemmPlanDesc d = fit_tile(desc);
+  const GemmPlanDesc d = settle(desc, sms);
   std::vector<std::string> bad;
   auto need = [&](const char* what, int64_t want, int64_t have, const char* unit) {
     if (have > 0 && want > have)
@@ -478,7 +514,11 @@ std::vector<std::string> plan_check(const GemmPlanDesc& desc, const PlanExtents&
 }
 
 int64_t gemm_plan_create(const GemmPlanDesc& desc) {
-  const GemmPlanDesc d = fit_tile(desc);
+  if (desc.K % 8 != 0) throw std::runtime_error("tridist_b200: K must be a multiple of 8");
+  if (desc.N % 8 != 0) throw std::runtime_error("tridist_b200: N must be a multiple of 8");
+  bool few;
+  SkinnyParams few_layout;
+  const GemmPlanDesc d = settle(desc, num_sms(), few, few_layout);
   if (d.R < 1 || d.R > kMaxRanks) throw std::runtime_error("tridist_b200: 1 <= R <= 8 required");
   if (d.bn != 128 && d.bn != 256) throw std::runtime_error("tridist_b200: BN must be 128 or 256");
   if (d.epi == EPI_SWIGLU && d.bn != 256)
@@ -503,8 +543,6 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
       if (d.mc_part[par] == 0 || d.mc_part[par] % 16 != 0)
         throw std::runtime_error("tridist_b200: switch-reduced reduce-scatter needs a 16-byte aligned multicast address");
   }
-  if (d.K % 8 != 0) throw std::runtime_error("tridist_b200: K must be a multiple of 8");
-  if (d.N % 8 != 0) throw std::runtime_error("tridist_b200: N must be a multiple of 8");
   auto* plan = new GemmPlan();
   plan->bn = d.bn;
   plan->bf16 = d.bf16;
@@ -586,9 +624,10 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
     p.env.rank = static_cast<uint32_t>(d.rank);
   }
   plan->grid_x = grid_for(d, plan->prm[0], d.max_ctas, num_sms());
-  plan->skinny = takes_few_rows(d, num_sms(), plan->few);
-  if (plan->skinny) {
+  plan->skinny = few;
+  if (few) {
     SkinnyParams& f = plan->few;
+    f = few_layout;
     if (f.swiglu) f.up_row0 = d.swiglu_up_row0;
     f.tma_a = make_tmap(reinterpret_cast<void*>(d.a), d.a_rows, d.K, d.lda, d.bf16, f.ar);
     f.tma_b = make_tmap(reinterpret_cast<void*>(d.b), d.b_rows, d.K, d.ldb, d.bf16, f.wr);

@@ -44,7 +44,7 @@ struct GemmPlanDesc {
   int allow_wide = 1;   // let CTA pairs take 512 x 256 tiles (256 rows per CTA) where the rows allow
   int allow_splitk = 1; // let the tiles of the last, partial scheduling round be cut along K
   int early_start = 1;  // one rank: the launch may start under the tail of the kernel in front of it
-  int few_rows = 0;     // one rank: the kernel of skinny_gemm.cuh for at most 128 rows, and for 256 where it is expected to be faster (2: for those too)
+  int few_rows = 0;     // one rank: the kernel of skinny_gemm.cuh for at most 256 rows, by the rule of settle() (2: wherever it can)
   double tile_us = 0;   // (the time that fit_tile expects)
   int fit_tile = 0;     // bn, pairs and the tile's height by the time expected of them (one rank; see fit_tile)
   int by_rounds = 0;    // tile height by the rounds it takes (local launches whose width is given; see choose_cta_mt)

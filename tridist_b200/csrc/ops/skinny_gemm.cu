@@ -73,12 +73,18 @@ static SkinnyParams lay_out(int M, int N, int K, bool swiglu, bool bf16, int sms
   return p;
 }
 
-SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms) {
+SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms, bool odd_rows) {
   // The expected time: B from DRAM; what a CTA loads in all, at about 120 GB/s through its L2 port, or its k-blocks,
   // 130 ns each however small; the two overlap, not wholly. A cluster starts later and exchanges parts, 2.5 us for
   // two CTAs and 5 for four. us measured with clusters of 1, 2 and 4 (rows x N x K): 128 x 8192 x 28672 89.5, 81.7 and 104;
   // 128 x 8192 x 3584 15.2, 16.6 and 23.7; 64 x 4096 x 1376 7.6, 8.4 and 9.3; 64 x 2048 x 16384 36.7, 25.7 and 21.3;
   // 128 x 512 x 8192 23.7, 15.9 and 15.5. 128 x 28672 x 8192 by shares of 104 and of 200 rows 92.7 and 76.8.
+  auto cta_us = [](const SkinnyParams& p, double port) {
+    const double mma = p.mb * 4 * std::max(p.mma_n, 48) / 2 / 1.7e3;        // us a k-block
+    const double rounds = ceil_div(p.shares, p.workers);
+    return rounds * (p.range.len + 1) * std::max({(p.ar + p.wr * p.boxes) * 128 / 0.12e6 * port, mma, 0.13});
+  };
+  const double dram = static_cast<double>(N) * (swiglu ? 2 : 1) * K * 2 / 6.3e6;
   SkinnyParams best;
   double best_us = -1;
   for (int cl2 = 0; 1 << cl2 <= kSkinnyMaxCluster; ++cl2)
@@ -87,20 +93,22 @@ SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms) {
       if (best_us >= 0 && (p.tmem_cols > 512 || p.smem_bytes > kSkinnySmem)) continue;
       if (cl2 > 0 && (p.range.len < 2 || p.shares > p.workers)) continue;     // (a cluster meets once)
       if (best_us >= 0 && p.stages * p.stage_bytes < 120 * 1024) continue;    // (too little in flight)
-      const double mma = p.mb * 4 * std::max(p.mma_n, 48) / 2 / 1.7e3;        // us a k-block
-      const double rounds = ceil_div(p.shares, p.workers);
-      const double dram = static_cast<double>(N) * p.boxes * K * 2 / 6.3e6;
-      const double cta = rounds * (p.range.len + 1) * std::max({(p.ar + p.wr * p.boxes) * 128 / 0.12e6, mma, 0.13});
-      const double us = std::max(dram, cta) + 0.3 * std::min(dram, cta) + (cl2 == 0 ? 0.0 : cl2 == 1 ? 2.5 : p.mb == 1 ? 5.0 : 9.0);
+      const double meet = cl2 == 0 ? 0.0 : cl2 == 1 ? 2.5 : p.mb == 1 ? 5.0 : 9.0;
+      const double cta = cta_us(p, 1.0);
+      const double us = std::max(dram, cta) + 0.3 * std::min(dram, cta) + meet;
       if (best_us < 0 || us < 0.98 * best_us) {
         best = p;
         best_us = us;
+        const double odd = odd_rows ? cta_us(p, 1.6) : cta;
+        best.us = std::max(dram, odd) + 0.3 * std::min(dram, odd) + meet;
       }
     }
   // With start and epilogue. Two blocks of A leave the ring three to five short stages: 12 % more. The tiles of the general
   // kernel are faster where they fill the device with a long K to cut. us here and there: 192 x 896 x 608 8.9 and 14.3,
   // 256 x 11008 x 4096 45 and 67, 192 x 29568 x 8192 109 and 132; 192 x 8192 x 28672 120 and 111.
-  best.us = (best_us + 4.0) * (best.mb == 2 ? 1.12 : 1.0);
+  // Rows on odd multiples of 16 bytes (`odd_rows`): a 128-byte piece of each lies in five sectors and two lines, and the
+  // port takes 1.6 times as long (median of 100 shapes of 40 to 256 rows); the layout stays.
+  best.us = (best.us + 4.0) * (best.mb == 2 ? 1.12 : 1.0);
   return best;
 }
 

@@ -54,8 +54,9 @@ struct SkinnyParams {
   WaitEnv env;
 };
 
-// Fills everything but the tensor maps, c, ldc and env. `sms`: CTAs that can run at once.
-SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms);
+// Fills everything but the tensor maps, c, ldc and env. `sms`: CTAs that can run at once; `odd_rows`: rows of an operand start
+// on odd multiples of 16 bytes (of the expected time only).
+SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms, bool odd_rows = false);
 // First and end group of every share.
 std::vector<std::array<int, 2>> skinny_shares(const SkinnyParams& p);
 void skinny_launch(const SkinnyParams& p, bool early_start, void* stream);
