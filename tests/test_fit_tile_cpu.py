@@ -39,3 +39,15 @@ def test_every_tile_once():
         kw = {k: int(v) for k, v in kw.items()}
         out, bad = _dump(**kw)
         assert bad == [] and len(out) <= 148, (kw, bad)
+
+
+@pytest.mark.parametrize("M,N,K,epi,bn,cta_m,row_blocks", [
+    (3589, 26240, 64, 0, 256, 2, 1), (1000, 12736, 800, 0, 256, 2, 1), (520, 24256, 608, 0, 256, 2, 1),
+    (1184, 17856, 80, 0, 256, 2, 1), (2312, 12304, 112, 1, 256, 1, 1), (1020, 3616, 336, 1, 256, 1, 1),
+])
+def test_choice_where_the_epilogue_is_longer_than_the_product(M, N, K, epi, bn, cta_m, row_blocks):
+    from tridist_b200.ops._gemm_common import OP_PLAIN, SCHED_NATURAL
+    from tridist_b200.parallel.runtime import native
+    got = native().gemm_choice(dict(op=OP_PLAIN, sched=SCHED_NATURAL, bn=256, R=1, rank=0, by_rounds=1, fit_tile=1, M=M, N=N,
+                                    K=K, epi=epi), 148)
+    assert (got["bn"], got["cta_m"], got["row_blocks"]) == (bn, cta_m, row_blocks)

@@ -183,18 +183,21 @@ static int row_alignment(const GemmPlanDesc& d) {
 // long runs under the power cap their operand traffic costs that much. us with 128 x 128, 128 x 256, 256 x 256 and 512 x 256
 // tiles (rows x N x K): 384 x 3328 x 1584 16.8, 23.6, 21.6, 25.2; 320 x 28672 x 8192 236, 160, 171, 171; 2112 x 22016 x
 // 4096 485, 316, 276, 314; 1728 x 12288 x 12288 656, 416, 370, 446; 8192 x 6144 x 12288 774 as 512 x 256, 800 as 256 x 256.
+// A round takes no less than its epilogue (`least`), which a K below 1000 does not cover; over 90 shapes of 140 to 8192 rows and
+// a K of 64 to 2200 the tile chosen is 0.7 % slower than the fastest on average, 11 % without it: 3589 x 26240 x 64 143, 108,
+// 77.5, 81, 1000 x 12736 x 800 37, 30, 24, 34, with SwiGLU 2312 x 2 x 12304 x 112 - , 99, 153, 143.
 // Rows on odd multiples of 16 bytes, which make every 128-byte piece of an operand lie in two lines, keep the given width and
 // the height by rounds: the constants were fitted without them, and the tiles they choose there move more operands (34
 // such shapes of 136 to 2000 rows: 1.7 % slower on average, up to 40 %).
 static GemmPlanDesc fit_tile(GemmPlanDesc d) {
   if (!d.fit_tile || d.R != 1 || d.sched != SCHED_NATURAL || d.max_ctas > 0 || d.probe != 0) return d;
-  struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi, energy; };
+  struct Tile { int bn, blocks, pairs; double per_kb, fixed, meet, epi, energy, least; };
   const bool swiglu = d.epi == EPI_SWIGLU;
-  const Tile tiles[4] = {{128, 1, 0, 0.375, 8.0, 5.0, 0.0, 1.45},
-                         {256, 1, 0, 0.47, 10.0, 6.5, 0.0, 1.2},
-                         {256, 2, 1, 0.42, 12.0, 6.0, 0.0, 1.07},
-                         {256, 4, 1, 0.78, 12.0, 12.0, swiglu ? 6.0 : 3.5, 1.0}};
   const int mt = (d.M + BM - 1) / BM, kb = (d.K + BK - 1) / BK;
+  const Tile tiles[4] = {{128, 1, 0, 0.375, 8.0, 5.0, 0.0, 1.45, 4.0},
+                         {256, 1, 0, 0.47, 10.0, 6.5, 0.0, 1.2, swiglu ? 4.0 : 6.0},
+                         {256, 2, 1, 0.42, std::min(12.0, 9.0 + 0.1 * kb), 6.0, 0.0, 1.07, swiglu ? 6.0 : 4.0},
+                         {256, 4, 1, 0.78, 12.0, 12.0, swiglu ? 6.0 : 3.5, 1.0, swiglu ? 10.0 : 7.0}};
   const double dram = (static_cast<double>(d.N) * (swiglu ? 2 : 1) * d.K + static_cast<double>(d.M) * (d.K + d.N)) * 2 / 6.3e6;
   const double power = 2.0 * d.M * d.N * (swiglu ? 2 : 1) * d.K / 1.25e9;
   double best_us = -1;
@@ -206,8 +209,8 @@ static GemmPlanDesc fit_tile(GemmPlanDesc d) {
     const int64_t n = static_cast<int64_t>((mt + t.blocks - 1) / t.blocks) * ((d.N + bn_out - 1) / bn_out);
     const int left = static_cast<int>(n % g), s = d.allow_splitk ? slices_for(left, g, kb) : 1;
     const double whole = kb * t.per_kb;
-    double us = static_cast<double>(n / g) * (whole + t.epi);
-    if (left > 0) us += (s == 1 ? whole : std::min(whole, whole / s + t.meet)) + t.epi;
+    double us = static_cast<double>(n / g) * std::max(whole + t.epi, t.least);
+    if (left > 0) us += std::max((s == 1 ? whole : std::min(whole, whole / s + t.meet)) + t.epi, t.least);
     us = std::max(std::max(us, dram) + t.fixed, power * t.energy);
     if (best_us >= 0 && us >= best_us) continue;
     best_us = us;
