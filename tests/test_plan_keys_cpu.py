@@ -12,8 +12,10 @@ class _Native:
     """Plans are numbered and their descriptors kept; nothing is launched."""
 
     def __init__(self):
+        from tridist_b200.parallel.runtime import native
         self.descs = {}
         self.launched = []
+        self.settings = native().settings
 
     def gemm_plan_create(self, d):
         self.descs[len(self.descs) + 1] = d
@@ -104,3 +106,36 @@ def test_forced_width_is_part_of_the_key(op, M, N, K, first, monkeypatch):
         assert d["bn"] == 256
         assert (d["fit_tile"], d["few_rows"]) == ((1, int(M <= 256)) if width is None else (0, 0)), (width, fake.launched)
     assert fake.launched == [1, 2, 1, 2]
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_one_look_at_the_environment_a_call(op, monkeypatch):
+    """A first call on new operands pays for every look-up."""
+    import os
+    from tridist_b200.ops import _gemm_common as common
+    fake = _Native()
+    looks = []
+    settings = fake.settings
+    fake.settings = lambda: looks.append(1) or settings()
+    call = _caller(op, 256, 4096, 1024, fake, monkeypatch)
+    asked = []
+    get = os.environ.get
+    monkeypatch.setattr(common, "env_int", lambda n, d: asked.append(n) or int(get(n) or d))
+    call()
+    assert looks == [1] and asked == []
+
+
+def test_settings_are_those_of_the_process(monkeypatch):
+    from tridist_b200.ops import _gemm_common as common
+    from tridist_b200.parallel.runtime import native
+    for name in list(native().settings()):
+        monkeypatch.delenv(name)
+    assert native().settings() == {} and common.plan_env() == common._PLAN_ENV
+    monkeypatch.setenv("TRIDIST_SPLITK", "0")
+    monkeypatch.setenv("TRIDIST_FORCE_BN", "")           # empty: the default
+    monkeypatch.setenv("TRIDIST_VERIFY_TOL", "2e-2")     # not a plan's
+    assert native().settings() == {"TRIDIST_SPLITK": "0", "TRIDIST_FORCE_BN": "", "TRIDIST_VERIFY_TOL": "2e-2"}
+    assert common.plan_env() == {**common._PLAN_ENV, "TRIDIST_SPLITK": 0}
+    monkeypatch.setenv("TRIDIST_FORCE_BN", "wide")
+    with pytest.raises(ValueError):
+        common.plan_env()

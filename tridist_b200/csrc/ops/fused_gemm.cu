@@ -555,6 +555,10 @@ int64_t gemm_plan_create(const GemmPlanDesc& desc) {
   plan->staging = uses_staging(d, plan->cta_m, plan->cta_mt);
   for (int par = 0; par < 2; ++par) {
     GemmParams& p = plan->prm[par];
+    if (par == 1 && d.R == 1) {        // (the parities differ in what is shared with peers)
+      p = plan->prm[0];
+      continue;
+    }
     std::memset(&p, 0, sizeof(p));
     fill_schedule_fields(d, plan->cta_m, plan->cta_mt, p);
     p.order_table = reinterpret_cast<const int32_t*>(d.order_table);

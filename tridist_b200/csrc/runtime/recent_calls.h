@@ -7,12 +7,12 @@
 
 #include <array>
 #include <cstdint>
-#include <cstdlib>
 #include <algorithm>
 #include <unordered_map>
 #include <vector>
 
 #include "../ops/fused_gemm.h"
+#include "environment.h"
 
 namespace tdb {
 
@@ -26,6 +26,7 @@ class RecentCalls {
     if (tile_forced()) return false;
     it->second.used = ++clock_;
     ++hits_;
+    drained_ = false;
     gemm_plan_launch(it->second.plan, round, static_cast<int>(round & 1u), 0, 0, stream);
     return true;
   }
@@ -39,11 +40,13 @@ class RecentCalls {
   void clear() { calls_.clear(); }
   // Keys of the plans launched from here since the last time, the least recent first.
   std::vector<pybind11::object> drain() {
+    std::vector<pybind11::object> out;
+    if (drained_) return out;
+    drained_ = true;
     std::vector<Call*> v;
     for (auto& c : calls_)
       if (c.second.used > 0) v.push_back(&c.second);
     std::sort(v.begin(), v.end(), [](const Call* x, const Call* y) { return x->used < y->used; });
-    std::vector<pybind11::object> out;
     for (Call* c : v) {
       out.push_back(c->cache_key);
       c->used = 0;
@@ -54,11 +57,12 @@ class RecentCalls {
 
  private:
   static bool tile_forced() {      // by the environment: the Python key, which such a call goes to, looks at it every time
-    for (const char* name : {"TRIDIST_FORCE_BN", "TRIDIST_MAX_CTAS"}) {
-      const char* v = std::getenv(name);
-      if (v != nullptr && *v != 0) return true;
-    }
-    return false;
+    bool forced = false;
+    each_setting([&](const char* name, size_t n, const char* value) {
+      forced = forced || (*value != 0 && n == 16 && (std::memcmp(name, "TRIDIST_FORCE_BN", 16) == 0 ||
+                                                     std::memcmp(name, "TRIDIST_MAX_CTAS", 16) == 0));
+    });
+    return forced;
   }
   static constexpr int kWords = 19;
   struct Key {
@@ -94,6 +98,7 @@ class RecentCalls {
   std::unordered_map<Key, Call, Hash> calls_;
   uint64_t clock_ = 0;
   int64_t hits_ = 0;
+  bool drained_ = true;      // nothing launched from here since the last drain
 };
 
 }  // namespace tdb

@@ -29,7 +29,7 @@ def is_bf16(dtype: torch.dtype) -> bool:
     raise TypeError(f"tridist_b200: fused GEMM kernels support fp16 and bf16, got {dtype}")
 
 
-def choose_bn(M: int, N: int, swiglu: bool = False, K: int = 0, local: bool = False) -> int:
+def choose_bn(M: int, N: int, swiglu: bool = False, K: int = 0, local: bool = False, env: Optional[Dict[str, int]] = None) -> int:
     """Output-tile width: 256 unless that leaves most SMs without a tile. A single row block
     (M <= 128) with a long K is the exception: every CTA re-reads the whole A slice of its K
     range, so wider tiles (fewer CTAs per K range, more K slices instead) move a quarter less
@@ -40,7 +40,7 @@ def choose_bn(M: int, N: int, swiglu: bool = False, K: int = 0, local: bool = Fa
     pick its tile itself (``fit_tile`` of the descriptor) takes this width only as part of its key."""
     if swiglu:
         return 256       # gate and up halves are two 128-row TMA boxes of one 256-wide tile
-    forced = env_int("TRIDIST_FORCE_BN", 0)
+    forced = env_int("TRIDIST_FORCE_BN", 0) if env is None else env["TRIDIST_FORCE_BN"]
     if forced in (128, 256):
         return forced
     m_tiles = (M + BM - 1) // BM
@@ -203,17 +203,33 @@ def read_prof(n_ctas: int = 148) -> Dict[str, Dict[str, float]]:
     return out
 
 
-def tile_is_free(world, R: int) -> bool:
+# What a plan takes from the environment, with its default.
+_PLAN_ENV = {"TRIDIST_MAX_CTAS": 0, "TRIDIST_FORCE_BN": 0, "TRIDIST_CHECK_RESIDENCY": 1, "TRIDIST_POLL_NS": 0, "TRIDIST_WIDE": 1,
+             "TRIDIST_SPLITK": 1, "TRIDIST_RASTER_G": 0, "TRIDIST_L2_AHEAD": 0, "TRIDIST_PROF": 0, "TRIDIST_CTA_PAIR": 1,
+             "TRIDIST_EMU_PAIR": 0, "TRIDIST_DEBUG": 0}
+
+
+def plan_env() -> Dict[str, int]:
+    """The environment of a plan in one look, which a call passes on: one for each name and use took 7 of the 37 us of a
+    first call on new operands."""
+    given = {n: int(v) for n, v in native().settings().items() if v and n in _PLAN_ENV}
+    return {**_PLAN_ENV, **given} if given else _PLAN_ENV
+
+
+def tile_is_free(world, R: int, env: Dict[str, int]) -> bool:
     """One rank: the tile (or, for few rows, the kernel) is the plan's own choice unless the environment makes it. Part
     of every plan's key: a forced width may be the one that the free choice would start from."""
-    return (R == 1 and getattr(world, "kind", "") != "emulated" and not env_int("TRIDIST_MAX_CTAS", 0) and
-            not env_int("TRIDIST_FORCE_BN", 0))
+    return (R == 1 and getattr(world, "kind", "") != "emulated" and not env["TRIDIST_MAX_CTAS"] and
+            not env["TRIDIST_FORCE_BN"])
 
 
 def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr: int, ldc: int,
-              M: int, N: int, K: int, bn: int, op: int) -> Dict:
+              M: int, N: int, K: int, bn: int, op: int, env: Optional[Dict[str, int]] = None) -> Dict:
     assert a.stride(1) == 1 and b.stride(1) == 1, "operands must be row-major with unit inner stride"
-    free = tile_is_free(world, R)
+    if env is None:
+        env = plan_env()
+    emulated = getattr(world, "kind", "") == "emulated"
+    free = tile_is_free(world, R, env)
     d = dict(op=op, epi=EPI_STORE, sched=SCHED_NATURAL, bn=bn, bf16=is_bf16(a.dtype), rank=rank, R=R,
              M=M, N=N, K=K, a=a.data_ptr(), a_rows=a.shape[0], lda=a.stride(0),
              b=b.data_ptr(), b_rows=b.shape[0], ldb=b.stride(0), c=c_ptr, ldc=ldc,
@@ -222,21 +238,19 @@ def base_desc(world, rank: int, R: int, a: torch.Tensor, b: torch.Tensor, c_ptr:
              peer_abort=world.peer_abort_words() if hasattr(world, "peer_abort_words") else [],
              timeout_ns=world.timeout_ns,
              # the grid must fit the device in one wave: its CTAs wait on one another
-             check_residency=1 if (env_int("TRIDIST_CHECK_RESIDENCY", 1) and getattr(world, "kind", "") != "emulated") else 0,
-             max_ctas=env_int("TRIDIST_MAX_CTAS", 0) or
-             (NUM_SMS_HINT // world.num_ranks if getattr(world, "kind", "") == "emulated" else 0),
-             poll_ns=env_int("TRIDIST_POLL_NS", 0),
-             allow_wide=env_int("TRIDIST_WIDE", 1), allow_splitk=env_int("TRIDIST_SPLITK", 1),
+             check_residency=1 if (env["TRIDIST_CHECK_RESIDENCY"] and not emulated) else 0,
+             max_ctas=env["TRIDIST_MAX_CTAS"] or (NUM_SMS_HINT // world.num_ranks if emulated else 0),
+             poll_ns=env["TRIDIST_POLL_NS"],
+             allow_wide=env["TRIDIST_WIDE"], allow_splitk=env["TRIDIST_SPLITK"],
              # (ranks that compute together keep the tiles their exchange was measured with)
              by_rounds=1 if R == 1 else 0,
              few_rows=1 if (free and M <= 256) else 0, fit_tile=1 if free else 0,
-             raster_g=env_int("TRIDIST_RASTER_G", 0),
-             l2_ahead=env_int("TRIDIST_L2_AHEAD", 0),
-             prof=(prof_buffer().data_ptr() if prof_buffer() is not None else 0),
+             raster_g=env["TRIDIST_RASTER_G"],
+             l2_ahead=env["TRIDIST_L2_AHEAD"],
+             prof=prof_buffer().data_ptr() if env["TRIDIST_PROF"] else 0,
              # several virtual ranks in one launch keep to single-CTA tiles unless TRIDIST_EMU_PAIR=1
              # asks for CTA pairs there too (a cooperative launch of clusters)
-             allow_pair=1 if (env_int("TRIDIST_CTA_PAIR", 1) and
-                              (getattr(world, "kind", "") != "emulated" or env_int("TRIDIST_EMU_PAIR", 0))) else 0)
+             allow_pair=1 if (env["TRIDIST_CTA_PAIR"] and (not emulated or env["TRIDIST_EMU_PAIR"])) else 0)
     return d
 
 
@@ -250,7 +264,7 @@ def debug_check(d: Dict, **extents) -> None:
     check every ticket index and buffer offset the kernel will compute against the sizes of the
     buffers it is given (a bounds check that cannot fault: nothing is launched). Raises
     ``TriDistError`` with one sentence per violation."""
-    if not env_int("TRIDIST_DEBUG", 0):
+    if not plan_env()["TRIDIST_DEBUG"]:
         return
     bad = native().plan_check(d, {k: int(v) for k, v in extents.items()}, 148)
     if bad:
@@ -304,14 +318,15 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     assert out.stride(1) == 1
     w = plain_world()
-    free = bn is None and local and not max_ctas and not probe and tile_is_free(w, 1)      # (the tile is nobody's choice)
+    env = plan_env()
+    free = bn is None and local and not max_ctas and not probe and tile_is_free(w, 1, env)      # (the tile is nobody's choice)
     if bn is None:
-        bn = choose_bn(M, N, swiglu, K=K, local=local and not max_ctas)    # (the rule counts on all SMs)
+        bn = choose_bn(M, N, swiglu, K=K, local=local and not max_ctas, env=env)    # (the rule counts on all SMs)
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
            out.stride(0), bn, swiglu, a.dtype, max_ctas, probe, local, free)
 
     def make():
-        d = base_desc(w, 0, 1, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_PLAIN)
+        d = base_desc(w, 0, 1, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_PLAIN, env)
         if swiglu:
             d["epi"] = EPI_SWIGLU
             d["swiglu_up_row0"] = N
@@ -322,7 +337,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
             d["few_rows"] = d["fit_tile"] = 0
         if not local:
             d["by_rounds"] = d["early_start"] = 0
-        debug_check(d, c_bytes=tensor_extent_bytes(out))
+        if env["TRIDIST_DEBUG"]:
+            debug_check(d, c_bytes=tensor_extent_bytes(out))
         return native().gemm_plan_create(d)
 
     pid = _plain_cache.get(key, make)

@@ -40,7 +40,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, EPI_SWIGLU, OP_AG, SCHED_NATURAL, SCHED_SEGMENT, PlanCache,
-                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
+                           base_desc, choose_bn, debug_check, rotation_order, plan_env, tensor_extent_bytes, tile_is_free)
 
 _CONSUMER_BLOCK_M = 128
 _CONSUMER_BLOCK_N = 128
@@ -247,17 +247,18 @@ def _plan(ctx, a, b, c, swiglu=False):
     M = m_pr * R
     n_rows = b.shape[0]
     N = n_rows // 2 if swiglu else n_rows
-    bn = choose_bn(M, N, swiglu, K=K, local=R == 1)
+    env = plan_env()
+    bn = choose_bn(M, N, swiglu, K=K, local=R == 1, env=env)
     order = ctx.order_override or rotation_order(rank, R, 1, own_last=False)
     # emulated launches cannot take a per-call table: a device order table is baked into the plan
     baked_table = getattr(ctx, "emu_order_table", None)
     key = (a.data_ptr(), b.data_ptr(), c.data_ptr(), m_pr, n_rows, K, a.stride(0), b.stride(0), c.stride(0),
            a.dtype, swiglu, bn, tuple(order), baked_table.data_ptr() if baked_table is not None else 0,
            ctx.observe, getattr(ctx, "emu_table_header", False), getattr(ctx, "seg_bands", 0), getattr(ctx, "seg_own_first", 0), ctx.transport,
-           ctx.push_ctas, tile_is_free(ctx.world, R))
+           ctx.push_ctas, tile_is_free(ctx.world, R, env))
 
     def make():
-        d = base_desc(ctx.world, rank, R, a, b, c.data_ptr(), c.stride(0), M, N, K, bn, OP_AG)
+        d = base_desc(ctx.world, rank, R, a, b, c.data_ptr(), c.stride(0), M, N, K, bn, OP_AG, env)
         d["a_rows"] = m_pr
         d["m_per_rank"] = m_pr
         # (one rank has one segment: the plain raster, which an odd number of row blocks does not
@@ -302,7 +303,7 @@ def _plan(ctx, a, b, c, swiglu=False):
                 d["peer_ag_arrive"] = ctx.arrive.ptrs()
             debug_check(d, c_bytes=tensor_extent_bytes(c), ws_bytes=ctx.max_M * K * 2,
                         ag_flag_words=ctx.flags.nbytes // 4)
-        else:
+        elif env["TRIDIST_DEBUG"]:
             debug_check(d, c_bytes=tensor_extent_bytes(c))
         return native().gemm_plan_create(d)
 

@@ -45,7 +45,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, OP_AR1, OP_AR2, OP_PLAIN, SCHED_STRIDED, PlanCache,
-                           base_desc, choose_bn, debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
+                           base_desc, choose_bn, debug_check, rotation_order, plan_env, tensor_extent_bytes, tile_is_free)
 
 
 @dataclass
@@ -179,7 +179,8 @@ def _plan(ctx, a, b, c, mode, parity):
     R, rank = ctx.num_ranks, ctx.rank
     M, K = a.shape
     N = b.shape[0]
-    bn = choose_bn(M, N, K=K if ctx.num_ranks == 1 else 0, local=R == 1)   # (wide tiles halve the CTAs that publish and reduce)
+    env = plan_env()
+    bn = choose_bn(M, N, K=K if ctx.num_ranks == 1 else 0, local=R == 1, env=env)   # (wide tiles halve the CTAs that publish and reduce)
     res_is_c = 0
     plane = ctx.max_M * ctx.N * 2
     if mode in ("two_shot", "nvls"):
@@ -187,12 +188,12 @@ def _plan(ctx, a, b, c, mode, parity):
             (ctx.mc.local_ptr + (2 + parity) * plane)
         res_is_c = 1 if (c.data_ptr() == res_ptr and c.stride(0) == N) else 0
     key = (a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, a.stride(0), b.stride(0), c.stride(0),
-           a.dtype, bn, mode, res_is_c, parity if res_is_c else -1, tile_is_free(ctx.world, R))
+           a.dtype, bn, mode, res_is_c, parity if res_is_c else -1, tile_is_free(ctx.world, R, env))
 
     def make():
         op = {"local": OP_PLAIN, "gemm": OP_PLAIN, "one_shot": OP_AR1, "two_shot": OP_AR2,
               "nvls": OP_AR2}[mode]
-        d = base_desc(ctx.world, rank, R, a, b, c.data_ptr(), c.stride(0), M, N, K, bn, op)
+        d = base_desc(ctx.world, rank, R, a, b, c.data_ptr(), c.stride(0), M, N, K, bn, op, env)
         if mode == "nvls":
             # partials stay here: every "slot" entry is this rank's own partial plane
             d["nvls"] = 1
@@ -224,12 +225,13 @@ def _plan(ctx, a, b, c, mode, parity):
                 d["peer_res"] = [ctx.res.ptrs(0), ctx.res.ptrs(plane)]
             d["peer_res_flags"] = ctx.res_flags.ptrs()
             d["res_is_c"] = res_is_c
-        ext = dict(c_bytes=tensor_extent_bytes(c))
-        if op in (OP_AR1, OP_AR2):
-            ext.update(slot_bytes=plane if mode == "nvls" else R * plane, tile_flag_words=ctx.tile_flags.nbytes // 4)
-        if op == OP_AR2:
-            ext.update(res_bytes=plane, res_flag_words=ctx.res_flags.nbytes // 4)
-        debug_check(d, **ext)
+        if env["TRIDIST_DEBUG"]:
+            ext = dict(c_bytes=tensor_extent_bytes(c))
+            if op in (OP_AR1, OP_AR2):
+                ext.update(slot_bytes=plane if mode == "nvls" else R * plane, tile_flag_words=ctx.tile_flags.nbytes // 4)
+            if op == OP_AR2:
+                ext.update(res_bytes=plane, res_flag_words=ctx.res_flags.nbytes // 4)
+            debug_check(d, **ext)
         return native().gemm_plan_create(d)
 
     pid = ctx.plans.get(key, make)

@@ -36,7 +36,7 @@ from ..parallel.runtime import (CpuWorld, EmulatedWorld, SymmBuffer, default_wor
                                 native)
 from ..utils.config import env_int, env_str
 from ._gemm_common import (next_round, BM, OP_RS, SCHED_NATURAL, SCHED_SEGMENT, PlanCache, base_desc, choose_bn,
-                           debug_check, rotation_order, tensor_extent_bytes, tile_is_free)
+                           debug_check, rotation_order, plan_env, tensor_extent_bytes, tile_is_free)
 
 
 @dataclass
@@ -153,15 +153,16 @@ def _plan(ctx, a, b, out):
     M, K = a.shape
     N = b.shape[0]
     m_pr = M // R
-    bn = choose_bn(M, N, K=K, local=R == 1)
+    env = plan_env()
+    bn = choose_bn(M, N, K=K, local=R == 1, env=env)
     mode = pick_mode(ctx, M)
     # through the switch all ranks walk the same order (lockstep over the owners' segments)
     order = list(range(R)) if mode == "nvls" else (ctx.order_override or rotation_order(rank, R, 1, own_last=True))
     key = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-           a.dtype, bn, tuple(order), mode, ctx.reduce_ctas, ctx.reduce_tail, tile_is_free(ctx.world, R))
+           a.dtype, bn, tuple(order), mode, ctx.reduce_ctas, ctx.reduce_tail, tile_is_free(ctx.world, R, env))
 
     def make():
-        d = base_desc(ctx.world, rank, R, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_RS)
+        d = base_desc(ctx.world, rank, R, a, b, out.data_ptr(), out.stride(0), M, N, K, bn, OP_RS, env)
         d["m_per_rank"] = m_pr
         d["sched"] = SCHED_SEGMENT if (R > 1 and m_pr % BM == 0) else SCHED_NATURAL
         d["seg_order"] = order
@@ -182,7 +183,7 @@ def _plan(ctx, a, b, out):
                 d["slot_stride"] = m_pr * N
             debug_check(d, c_bytes=tensor_extent_bytes(out), slot_bytes=half,
                         tile_flag_words=ctx.tile_flags.nbytes // 4)
-        else:
+        elif env["TRIDIST_DEBUG"]:
             debug_check(d, c_bytes=tensor_extent_bytes(out))
         return native().gemm_plan_create(d)
 
