@@ -68,3 +68,20 @@ def test_alignment_is_that_of_addresses_and_strides(part):
 def test_sizes_that_a_plan_refuses_are_not_laid_out():
     for kw in (dict(M=64, N=0, K=64), dict(M=0, N=64, K=64), dict(M=64, N=64, K=0), dict(M=64, N=4, K=64)):
         assert not _choice(**kw)["few_rows"]
+
+
+def test_stall_accounting_does_not_change_the_kernel():
+    """What is timed beside the accounting is the kernel of other runs."""
+    for M in (16, 128, 192):
+        kw = dict(M=M, N=4096, K=1376)
+        assert _choice(prof=4096, **kw) == _choice(**kw) and _choice(**kw)["few_rows"]
+
+
+def test_a_plane_that_no_kernel_wrote_gives_no_accounting(monkeypatch):
+    import torch
+    from tridist_b200.ops import _gemm_common as common
+    plane = torch.zeros((256, common.PROF_WIDTH), dtype=torch.int64)
+    monkeypatch.setattr(common, "_prof_buf", plane)
+    assert common.read_prof() == {}
+    plane[3, 9] = 5000
+    assert common.read_prof()["kernel"]["max"] == 5.0

@@ -247,7 +247,7 @@ static bool uses_staging(const GemmPlanDesc& d, int cta_m, int cta_mt) {
 static GemmPlanDesc settle(const GemmPlanDesc& desc, int sms, bool& few, SkinnyParams& f) {
   GemmPlanDesc d = fit_tile(desc);
   few = false;
-  if (!d.few_rows || d.R != 1 || d.sched != SCHED_NATURAL || d.M < 1 || d.M > 256 || d.N < 8 || d.K < 8 || d.prof != 0 || d.c % 16 != 0 || d.ldc % 8 != 0)
+  if (!d.few_rows || d.R != 1 || d.sched != SCHED_NATURAL || d.M < 1 || d.M > 256 || d.N < 8 || d.K < 8 || d.c % 16 != 0 || d.ldc % 8 != 0)
     return d;
   const int align = row_alignment(d);
   f = skinny_plan(d.M, d.N, d.K, d.epi == EPI_SWIGLU, d.bf16, sms, align < 32);

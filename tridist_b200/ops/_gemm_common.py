@@ -184,10 +184,13 @@ def prof_buffer() -> Optional[torch.Tensor]:
 
 def read_prof(n_ctas: int = 148) -> Dict[str, Dict[str, float]]:
     """Mean and max over CTAs of every accounting slot of the LAST kernel, in microseconds
-    (``epi_tiles`` is a count). Call after a synchronisation."""
+    (``epi_tiles`` is a count). Call after a synchronisation, on a plane that was zero before the kernel: the few-rows
+    kernel keeps no accounting, a plane that stayed zero gives an empty dict."""
     if _prof_buf is None:
         return {}
     t = _prof_buf[:n_ctas].cpu().double()
+    if not bool(t.any()):
+        return {}
     out = {}
     for i, name in enumerate(PROF_SLOTS):
         col = t[:, i]

@@ -29,7 +29,8 @@ TRIDIST_DEBUG             1: before a plan is created, replay its tile schedule 
                           ticket index and buffer offset against the buffers' sizes (nothing is launched)
 TRIDIST_CHECK_RESIDENCY   0: skip the check at plan creation that the whole grid of a kernel whose CTAs wait on
                           peers can be resident at once (default 1)
-TRIDIST_PROF              1: collect per-CTA stall accounting of the fused GEMM kernels
+TRIDIST_PROF              1: collect per-CTA stall accounting of the fused GEMM kernels (the few-rows kernel of one
+                          rank keeps none; TRIDIST_FORCE_BN accounts for the general kernel in its place)
 TRIDIST_AR_MODE           "auto" | "one_shot" | "two_shot" | "nvls"
 TRIDIST_AR_ONE_SHOT_BYTES size threshold (bytes of one rank's partial) below which
                           the one-shot all-reduce is used (default 4 MiB; peer-store algorithms)
