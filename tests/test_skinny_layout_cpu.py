@@ -42,3 +42,27 @@ def test_layout_holds_for_every_shape(seed):
         assert p["mb"] * bufs * p["accs"] * p["acc_cols"] <= p["tmem_cols"] <= 512 and p["tmem_cols"] & (p["tmem_cols"] - 1) == 0, what
         assert 1 <= p["accs"] <= max(1, min(ranges) // 16), what
         assert p["accs"] <= -(-min(ranges) // p["kw"]), what
+
+
+@pytest.mark.parametrize("instead", [dict(shares=140), dict(k_blocks=200), dict(wr=8), dict(ar=64), dict(own=0), dict(stages=17),
+                                     dict(pad=-20000), dict(smem_bytes=4096), dict(smem_bytes=226 * 1024), dict(tmem_cols=32)])
+def test_checked_mode_names_what_a_layout_would_miss(instead):
+    """TRIDIST_DEBUG=1 looks at the layout that runs, as well as at the schedule of the calls that it does not take."""
+    from tridist_b200.parallel.runtime import native
+    C, shape = native(), (128, 4096, 12288, False)
+    assert C.skinny_check(*shape, {}) == []
+    bad = C.skinny_check(*shape, instead)
+    assert bad and all(s.startswith("few-rows layout: ") for s in bad), bad
+
+
+def test_checked_mode_passes_what_plans_make():
+    from tridist_b200.ops._gemm_common import OP_PLAIN, SCHED_NATURAL
+    from tridist_b200.parallel.runtime import native
+    rnd = random.Random(9)
+    for _ in range(200):
+        M, N, K = rnd.randint(1, 256), 8 * rnd.randint(1, rnd.choice([4, 300, 2400])), 8 * rnd.randint(1, rnd.choice([20, 4000]))
+        d = dict(op=OP_PLAIN, sched=SCHED_NATURAL, bn=256, R=1, rank=0, M=M, N=N, K=K, ldc=N, epi=rnd.randint(0, 1), few_rows=2,
+                 fit_tile=1, by_rounds=1)
+        assert native().gemm_choice(d, 148)["few_rows"]
+        assert native().plan_check(d, dict(c_bytes=M * N * 2), 148) == [], d
+        assert native().plan_check(d, dict(c_bytes=M * N * 2 - 2), 148) != [], d

@@ -432,8 +432,11 @@ std::vector<std::array<int, 6>> splitk_dump(const GemmPlanDesc& desc, int sms) {
 }
 
 std::vector<std::string> plan_check(const GemmPlanDesc& desc, const PlanExtents& e, int sms) {
-  const GemmPlanDesc d = settle(desc, sms);
+  bool few;
+  SkinnyParams few_layout;
+  const GemmPlanDesc d = settle(desc, sms, few, few_layout);
   std::vector<std::string> bad;
+  if (few) bad = skinny_check(few_layout);      // (the schedule below is that of the calls which it does not take)
   auto need = [&](const char* what, int64_t want, int64_t have, const char* unit) {
     if (have > 0 && want > have)
       bad.push_back(std::string(what) + " needs " + std::to_string(want) + " " + unit + ", has " +

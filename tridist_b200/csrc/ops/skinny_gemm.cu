@@ -118,6 +118,33 @@ std::vector<std::array<int, 2>> skinny_shares(const SkinnyParams& p) {
   return out;
 }
 
+std::vector<std::string> skinny_check(const SkinnyParams& p) {
+  std::vector<std::string> bad;
+  auto need = [&](bool ok, const char* what) {
+    if (!ok) bad.push_back(std::string("few-rows layout: ") + what);
+  };
+  const int cluster = 1 << p.cluster_log2;
+  need(cluster <= kSkinnyMaxCluster && p.workers >= 1 && p.workers <= p.shares && (cluster == 1 || p.workers == p.shares),
+       "workers and shares");
+  need(p.share.start(p.shares) == p.groups && p.groups * 8 == p.N, "the shares do not cover the columns");
+  need(p.range.start(cluster) == p.k_blocks && p.range.len >= 1, "the ranges do not cover K");
+  const int most = p.share.len + (p.share.more > 0 ? 1 : 0);
+  need(p.share.len >= 1 && most * 8 <= p.wr && p.wr <= p.nb && p.wr <= 256, "a share is larger than its box");
+  need(p.M <= p.ar && p.ar <= 256 && p.M <= 32 * p.warps && p.M <= 128 * p.mb, "rows outside the boxes of A");
+  need(ceil_div(most, cluster) <= p.own, "a CTA adds up more groups than its parts have room for");
+  const int block = (p.ar + p.nb * p.boxes) * 128;
+  const int parts = (cluster - 1) * p.boxes * p.own * p.warps * 1024;
+  const int ring = p.stages * p.stage_bytes + p.pad;
+  need(p.stages >= 1 && p.stages <= kSkinnyMaxStages && p.stage_bytes >= p.kw * block, "stages of the ring");
+  need((p.parts_in_ring ? std::max(ring, parts) : ring + parts) <= p.smem_bytes && p.smem_bytes <= kSkinnySmem, "shared memory");
+  // (the MMA reads whole 128-row blocks of A: the last k-block's end in the columns of B and the pad)
+  need((p.kw - 1) * p.ar * 128 + p.mb * 128 * 128 <= p.stage_bytes + p.pad, "the MMA reads behind the ring");
+  const int bufs = p.shares > p.workers ? 2 : 1;
+  need(p.mma_n <= p.acc_cols && p.mma_n <= 256 && (p.mb * bufs * p.acc_cols << p.accs_log2) <= p.tmem_cols && p.tmem_cols <= 512,
+       "tensor memory");
+  return bad;
+}
+
 template <int kW>
 static void launch(const SkinnyParams& p, bool early_start, cudaStream_t stream) {
   auto* kernel = skinny_gemm_kernel<kW>;

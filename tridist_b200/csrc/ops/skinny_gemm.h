@@ -4,6 +4,7 @@
 
 #include <array>
 #include <cstdint>
+#include <string>
 #include <vector>
 
 #include "../common/status.h"
@@ -59,6 +60,8 @@ struct SkinnyParams {
 SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms, bool odd_rows = false);
 // First and end group of every share.
 std::vector<std::array<int, 2>> skinny_shares(const SkinnyParams& p);
+// What a layout would read or write outside the memory that it is given, one sentence each (for the checked mode).
+std::vector<std::string> skinny_check(const SkinnyParams& p);
 void skinny_launch(const SkinnyParams& p, bool early_start, void* stream);
 
 }  // namespace tdb
