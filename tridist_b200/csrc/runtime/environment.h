@@ -11,7 +11,8 @@ namespace tdb {
 template <typename F>
 void each_setting(F f) {
   for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
-    if (std::strncmp(*e, "TRIDIST_", 8) != 0) continue;
+    // (two characters in front of the call: repeated launches look through the environment too)
+    if ((*e)[0] != 'T' || (*e)[1] != 'R' || std::strncmp(*e, "TRIDIST_", 8) != 0) continue;
     const char* eq = std::strchr(*e, '=');
     if (eq != nullptr) f(*e, static_cast<size_t>(eq - *e), eq + 1);
   }
