@@ -993,7 +993,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
             if constexpr (kCtaM == 2) {
               // the leader's barrier collects the bytes of both CTAs' loads
               if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * TS::kStageBytes);
-  #pragma unroll
+#pragma unroll
               for (int h = 0; h < kMT; ++h)
                 tma_load_2d_pair(sa + h * (BM * BK * 2), amap, &full_bar[stage], kb * BK, a_row + h * BM);
               tma_load_2d_pair(sb, bmap, &full_bar[stage], kb * BK, b_row_pair);
@@ -1006,7 +1006,7 @@ fused_gemm_kernel(const __grid_constant__ GemmParams p0, const GemmParams* __res
                 tma_load_2d(sb + (BN / 2) * BK * 2, bmap, &full_bar[stage], kb * BK,
                             up_row0 + t.n_tile * (BN / 2));
               } else {
-  #pragma unroll
+#pragma unroll
                 for (int h = 0; h < BN / 128; ++h)
                   tma_load_2d(sb + h * 128 * BK * 2, bmap, &full_bar[stage], kb * BK, n0 + h * 128);
               }

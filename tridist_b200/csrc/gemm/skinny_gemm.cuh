@@ -1,6 +1,6 @@
 // C = A @ B^T for few rows of A (at most 256, a decode batch): the time is that of reading B once.
 //
-// A worker is a cluster of 1, 2, 4 or 8 CTAs. It takes a share of B's rows, an even run of 8-row groups, whole, and
+// A worker is a cluster of 1, 2 or 4 CTAs. It takes a share of B's rows, an even run of 8-row groups, whole, and
 // its CTAs a range of K each. Rows of A are re-read through L2 by every worker; what a CTA reads in all bounds
 // the cluster's size from below and its width from above (see skinny_plan). The CTAs hand one another the parts of their
 // sums in shared memory, each adds up a run of the share's groups in the order of the K ranges and stores it:
@@ -11,8 +11,8 @@
 // 1376 14.7 and 7.6, 128 x 8192 x 3584 23 and 15.5, 128 x 2 x 3584 x 8192 with SwiGLU 35.6 and 29.
 //
 // Roles (224 threads): warp 0 loads B, warp 6 A, warp 1 multiplies and owns the tensor memory, warps 2-5 store,
-// one TMEM lane quarter (32 rows) each of every 128-row block of A. A long range of K is summed in up to four accumulators, one run of it each, that
-// the epilogue adds in order. Loads and MMAs are issued by an elected lane of a warp whose control flow is
+// one TMEM lane quarter (32 rows) each of every 128-row block of A. A long range of K is summed in up to four
+// accumulators, one run of it each, that the epilogue adds in order. Loads and MMAs are issued by an elected lane of a warp whose control flow is
 // uniform, with a stage of kW k-blocks unrolled: a k-block is 32 to 128 cycles of the tensor pipe for so few
 // rows, and a loop that issues it from one diverged lane takes 400 or more.
 #pragma once
@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(kSkinnyThreads, 1) skinny_gemm_kernel(const __
             const int lo = owned(dst), hi = owned(dst + 1);
             for (int m = 0; m < p.mb && m * 4 + q < p.warps; ++m) {
               const uint32_t t = t0 + static_cast<uint32_t>(m * accs * acc_cols);
-              const uint32_t base = cluster_smem_addr(xbuf + (sub < dst ? sub : sub - 1) * x_src + (m * 128 + q * 32 + lane) * 16, static_cast<uint32_t>(dst));
+              const uint32_t base =
+                  cluster_smem_addr(xbuf + (sub < dst ? sub : sub - 1) * x_src + (m * 128 + q * 32 + lane) * 16, static_cast<uint32_t>(dst));
               for (int h = 0; h < (swiglu ? 2 : 1); ++h) {
                 auto send = [&](int g, auto& x) {
                   take(t, h * up_col + g * 8, x);

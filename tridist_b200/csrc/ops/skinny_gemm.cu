@@ -76,7 +76,8 @@ static SkinnyParams lay_out(int M, int N, int K, bool swiglu, bool bf16, int sms
 SkinnyParams skinny_plan(int M, int N, int K, bool swiglu, bool bf16, int sms, bool odd_rows) {
   // The expected time: B from DRAM; what a CTA loads in all, at about 120 GB/s through its L2 port, or its k-blocks,
   // 130 ns each however small; the two overlap, not wholly. A cluster starts later and exchanges parts, 2.5 us for
-  // two CTAs and 5 for four. us measured with clusters of 1, 2 and 4 (rows x N x K): 128 x 8192 x 28672 89.5, 81.7 and 104;
+  // two CTAs and 5 for four. us measured with clusters of 1, 2 and 4 (rows x N x K), back to back over one set of operands, the
+  // 126 MB of L2 clean (over changing inputs the first takes 87, behind 256 MB of writes 99): 128 x 8192 x 28672 89.5, 81.7 and 104;
   // 128 x 8192 x 3584 15.2, 16.6 and 23.7; 64 x 4096 x 1376 7.6, 8.4 and 9.3; 64 x 2048 x 16384 36.7, 25.7 and 21.3;
   // 128 x 512 x 8192 23.7, 15.9 and 15.5. 128 x 28672 x 8192 by shares of 104 and of 200 rows 92.7 and 76.8.
   auto cta_us = [](const SkinnyParams& p, double port) {

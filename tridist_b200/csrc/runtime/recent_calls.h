@@ -1,7 +1,7 @@
 // Calls of one rank whose plan is known: the operands are compared with those of earlier calls and the plan is
 // launched without a way back through Python's checks and key (a 64 x 4096 x 1376 call took 12.7 us on the host, its
 // kernel 7.6). A key holds everything that those checks and the plan depend on: addresses, sizes, strides, types and
-// devices of the three tensors, and the caller's tag. The plans stay the Python cache's, which drops them here too.
+// devices of the three tensors, and the caller's tag; while the environment forces the tile, calls go to the Python key. The plans stay the Python cache's, which drops them here too.
 #pragma once
 #include <torch/extension.h>
 
@@ -30,7 +30,8 @@ class RecentCalls {
     gemm_plan_launch(it->second.plan, round, static_cast<int>(round & 1u), 0, 0, stream);
     return true;
   }
-  void remember(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, int64_t plan, pybind11::object cache_key) {
+  void remember(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, int64_t tag, int64_t plan,
+                pybind11::object cache_key) {
     Key k;
     if (!tile_forced() && key_of(a, b, c, tag, k)) calls_[k] = Call{plan, 0, std::move(cache_key)};
   }

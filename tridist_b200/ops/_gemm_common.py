@@ -37,7 +37,9 @@ def choose_bn(M: int, N: int, swiglu: bool = False, K: int = 0, local: bool = Fa
 
     ``local`` (one rank): 256 as well where the K split of the CTA pairs' tiles fills three quarters
     of the 74 pairs (256 rows, K 8192, N 8192: 47 us on 64 pairs, 74 us on 128 tiles of 128 x 128). A plan that may
-    pick its tile itself (``fit_tile`` of the descriptor) takes this width only as part of its key."""
+    pick its tile itself (``fit_tile`` of the descriptor) keeps this width where rows start on odd multiples of 16
+    bytes, and where at most 128 rows are left to the general kernel; under a probe, TRIDIST_MAX_CTAS or a forced
+    width nothing else decides."""
     if swiglu:
         return 256       # gate and up halves are two 128-row TMA boxes of one 256-wide tile
     forced = env_int("TRIDIST_FORCE_BN", 0) if env is None else env["TRIDIST_FORCE_BN"]

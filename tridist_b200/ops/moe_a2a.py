@@ -11,9 +11,9 @@ Public API follows the reference (triton_dist/kernels/dcu/moe_a2a.py:287-555):
 * ``moe_combine_intra_node_op(ctx, topk_idx, output, topk_weights=None)``:
   ``output[t] = sum_j w[t, j] * out_{rank(e_j)}[scatter_idx[t, j]]`` in fp32.
 
-Per round: three kernels (metadata, dispatch, combine), no host synchronisation
-and no host-issued copy; completion of the dispatch kernel means every rank's
-rows have landed.
+Per round: three kernels (metadata, dispatch, combine; one rank's small batches take
+metadata and dispatch in one), no host synchronisation and no host-issued copy;
+completion of the dispatch kernel means every rank's rows have landed.
 """
 from __future__ import annotations
 
